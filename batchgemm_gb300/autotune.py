@@ -88,10 +88,15 @@ def measure(mode, cfg, K, slots, waves=6, reps=5, hbm_gbs=6000.0):
     ta = max(1, min(8, 1024 // bm))
     tb = max(1, min(8, 1024 // bn))
     tiles_per = ta * tb
-    n = max(1, -(-waves * slots // tiles_per))
+    # the SIMT kernel runs eight warp tiles side by side in a CTA; its leading
+    # dimensions are odd, as three in four arbitrary sizes are not multiples of 4
+    simt_warp = mode == "simt" and cfg < 7
+    n = max(1, -(-waves * slots * (8 if simt_warp else 1) // tiles_per))
     ra, rb = bm * ta, bn * tb
     M, N = (rb, ra) if swap else (ra, rb)
-    db = DeviceBatch([M] * n, [N] * n, [K] * n).fill_fast("normal", 0)
+    pad = 1 if mode == "simt" else 0
+    db = DeviceBatch([M] * n, [N] * n, [K] * n, lda=[M + pad] * n, ldb=[K + pad] * n,
+                     ldc=[M + pad] * n).fill_fast("normal", 0)
     with db.plan(mode, force_tile_config=cfg, rebalance=False) as p:
         info = p.info()
         assert info["num_tiles"] == n * tiles_per, (info["num_tiles"], n * tiles_per)

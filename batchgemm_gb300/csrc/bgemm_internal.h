@@ -43,20 +43,35 @@ struct TileItem {
 };
 
 // ---------------------------------------------------------------- SIMT ----
-// Tile configurations of the FP32 SIMT kernel: 256 threads arranged 16 x 16,
-// each owning a TM x TN register tile.
+// Tile configurations of the FP32 SIMT kernel.  The 128 x 128 tile (id 7) and
+// the thin ones (ids 8 and 9, for M <= 8 and N <= 8) are computed by a CTA of
+// 256 threads, the others by one warp (eight run side by side in a CTA): ids 1
+// to 6 as 32 x 32 parts in turn.
 struct SimtCfg {
-  int bm, bn, tm, tn;
+  int bm, bn;  // tile
+  int lm, ln;  // log2 of these
+  int gm, gn;  // steps in which a ragged edge's outputs are skipped
 };
-// Ids 8 and 9 are the thin tiles: 8 x 128 for M <= 8 (each thread four rows
-// of one column) and 128 x 8 for N <= 8 (one row of four columns), where the
-// 16-wide tiles would compute mostly padding.
 constexpr int kSimtNumCfgs = 10;
 constexpr SimtCfg kSimtCfgs[kSimtNumCfgs] = {
-    {16, 16, 1, 1},  {32, 32, 2, 2},  {64, 32, 4, 2},  {32, 64, 2, 4},
-    {64, 64, 4, 4},  {128, 64, 8, 4}, {64, 128, 4, 8}, {128, 128, 8, 8},
-    {8, 128, 4, 1},  {128, 8, 1, 4},
+    {16, 16, 4, 4, 16, 16},  {32, 32, 5, 5, 16, 16},  {64, 32, 6, 5, 16, 16},
+    {32, 64, 5, 6, 16, 16},  {64, 64, 6, 6, 16, 16},  {128, 64, 7, 6, 16, 16},
+    {64, 128, 6, 7, 16, 16}, {128, 128, 7, 7, 32, 16}, {8, 128, 3, 7, 8, 16},
+    {128, 8, 7, 3, 16, 8},
 };
+__host__ __device__ constexpr bool simt_warp_cfg(int cfg) { return cfg < 7; }
+// What the planners choose from: ids 2 to 6 run only when forced (their parts
+// in turn are no faster than tiles of their own); a thin matrix takes a thin
+// tile or, where even that is mostly padding, 16 x 16 ones (K = 4096 and M or
+// N <= 8, two batches of about 100 each: 568 and 474 us in thin tiles, 664 and
+// 610 in 16 x 16, 857 and 875 in 32 x 32).
+__host__ __device__ constexpr bool simt_auto_cfg(int cfg, int M, int N) {
+  return cfg == 0 || (cfg == 8 ? M <= 8 : cfg == 9 ? N <= 8
+                                                   : (cfg == 1 || cfg == 7) && M > 8 && N > 8);
+}
+// ids 1 to 6: 32-row and 32-column parts of a tile (one hex digit each)
+__host__ __device__ constexpr int simt_part_rows(int cfg) { return (0x2421210 >> (4 * cfg)) & 15; }
+__host__ __device__ constexpr int simt_part_cols(int cfg) { return (0x4222110 >> (4 * cfg)) & 15; }
 
 struct SimtParams {
   const MatDesc* descs;
@@ -70,9 +85,9 @@ struct SimtParams {
   float* const* C;
 };
 
-// transposed: the plan's matrices carry kTransAFlag / kTransBFlag
-cudaError_t simt_launch(const SimtParams& p, int grid, cudaStream_t stream,
-                        bool transposed = false);
+// ta / tb: the plan's matrices carry kTransAFlag / kTransBFlag
+cudaError_t simt_launch(const SimtParams& p, int grid, cudaStream_t stream, bool ta = false,
+                        bool tb = false);
 int simt_ctas_per_sm();
 
 }  // namespace bgemm

@@ -6,17 +6,15 @@
 //
 // Because the sizes live on the device, the tile queue is built there too:
 //   1. fw_plan_kernel (one CTA) picks each matrix's SIMT tile configuration
-//      with the same cost model as the host planner, rebalances for
-//      parallelism (the host planner's rule, in rounds: a matrix whose tile
-//      is longer than the average load of a persistent CTA moves to smaller
-//      tiles when that lowers the makespan bound), buckets matrices by
-//      modelled tile time (quarter-octave bins) and reserves each matrix a
+//      with the host planner's model and rule (tile_table.h), buckets matrices
+//      by modelled tile time (quarter-octave bins) and reserves each matrix a
 //      contiguous range of the queue, longest tiles first;
 //   2. fw_expand_kernel writes the work items (one warp per matrix);
 //   3. the persistent SIMT kernel reads the item count from the device.
 // The three launches allocate nothing and can be captured in a CUDA graph;
 // the queue scratch is owned by the library (one buffer per device, grown
 // when a call needs more).
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 #include <vector>
@@ -30,6 +28,7 @@ namespace bgemm {
 namespace {
 
 constexpr int kBins = 64;
+constexpr int kPlanThreads = 1024;
 
 __constant__ SimtCfg c_cfgs[kSimtNumCfgs];
 __constant__ TileCost c_cost[kSimtNumCfgs];
@@ -43,141 +42,91 @@ struct FwScratch {
   TileItem* items;  // [cap_items]
 };
 
-// One matrix's tile configuration and bin (the same cost model as the host
-// planner); shared by fw_plan_kernel and its host replay.  Tile times are
-// formed with one fmaf and work is summed as 64-bit integer nanoseconds, so
-// the device and the host replay (on any CPU) make the same decisions.
-struct FwMat {
-  int bad;    // size negative or above max_dim: skipped
-  int cfg;    // -1: no output (M or N is 0, or skipped)
-  int tiles;
-  int bin;    // quarter-octave bin of the modelled tile time
-};
-
-__host__ __device__ inline long long fw_tiles(int M, int N, const SimtCfg& g) {
-  return (long long)((M + g.bm - 1) / g.bm) * ((N + g.bn - 1) / g.bn);
+// A size that is negative or above max_dim: the matrix is skipped.
+__host__ __device__ inline bool fw_bad(int M, int N, int K, int max_dim) {
+  return M < 0 || N < 0 || K < 0 || M > max_dim || N > max_dim;
 }
-__host__ __device__ inline float fw_tile_ns(int K, const TileCost& c) {
-  return fmaf(c.b_ns, (float)K, c.a_ns);
-}
-// TileItem holds 16-bit tile coordinates: a configuration with more than
-// 65535 tiles along M or N is not a candidate (the host planner's rule).
-__host__ __device__ inline bool fw_fits(int M, int N, const SimtCfg& g) {
-  return (M + g.bm - 1) / g.bm <= 65535 && (N + g.bn - 1) / g.bn <= 65535;
-}
-__host__ __device__ inline long long fw_work(int M, int N, int K, int cfg, const SimtCfg* cfgs,
-                                             const TileCost* cost) {
-  return fw_tiles(M, N, cfgs[cfg]) * (long long)fw_tile_ns(K, cost[cfg]);
+__host__ __device__ inline int fw_bin(int K, TileCost t) {
+  const int q = quarter_octave(simt_tile_ns(K, t)) - 24;
+  return q < 0 ? 0 : q > kBins - 1 ? kBins - 1 : q;
 }
 
-__host__ __device__ inline FwMat fw_plan_matrix(int M, int N, int K, int max_dim,
-                                                const SimtCfg* cfgs, const TileCost* cost) {
-  FwMat r{};
-  r.bad = M < 0 || N < 0 || K < 0 || M > max_dim || N > max_dim;
-  r.cfg = -1;
-  if (!r.bad && M > 0 && N > 0) {
-    double bw = 0.0;
-    for (int c = kSimtNumCfgs - 1; c >= 0; --c) {
-      if (!fw_fits(M, N, cfgs[c])) continue;
-      const long long t = fw_tiles(M, N, cfgs[c]);
-      const double w = (double)t * fw_tile_ns(K, cost[c]);
-      if (r.cfg < 0 || w < bw * 0.999) {
-        r.cfg = c;
-        r.tiles = (int)t;
-        bw = w;
-      }
-    }
-  }
-  return r;
-}
-
-// Rebalance step of one matrix on configuration `cfg` (the host planner's
-// rule, plan.cpp choose_tiles): if its tile is longer than the average load
-// W / slots of a persistent CTA, the configuration with shorter and more
-// tiles of least total work, if that lowers the makespan bound
-// max(W / slots, longest tile) by at least a quarter; else -1.  (Measured on
-// the reference's shape file: the model overstates what splitting gains --
-// 4.8x predicted, 1.46x measured at 8 matrices -- and a 6 % predicted gain at
-// 256 matrices was a 7 % loss, hence the margin.)
-__host__ __device__ inline int fw_rebalance(int M, int N, int K, int cfg, long long W,
-                                            long long slots, const SimtCfg* cfgs,
-                                            const TileCost* cost) {
-  const long long tt = (long long)fw_tile_ns(K, cost[cfg]);
-  if (tt * slots <= W) return -1;
-  const long long tiles = fw_tiles(M, N, cfgs[cfg]);
-  const long long w_old = tiles * tt;
-  int best = -1;
-  long long bw = 0, btt = 0;
-  for (int c = 0; c < kSimtNumCfgs; ++c) {
-    if (!fw_fits(M, N, cfgs[c])) continue;
-    const long long t2 = (long long)fw_tile_ns(K, cost[c]);
-    const long long n2 = fw_tiles(M, N, cfgs[c]);
-    if (t2 >= tt || n2 <= tiles) continue;
-    const long long w = n2 * t2;
-    if (best < 0 || w < bw) {
-      best = c;
-      bw = w;
-      btt = t2;
-    }
-  }
-  if (best < 0) return -1;
-  const long long w_new = W - w_old + bw;
-  const long long before = W > tt * slots ? W : tt * slots;
-  const long long after = w_new > btt * slots ? w_new : btt * slots;
-  return after < before - before / 4 ? best : -1;
-}
-constexpr int kRebalanceRounds = 8;
-
-__global__ void fw_plan_kernel(const int* __restrict__ dM, const int* __restrict__ dN,
-                               const int* __restrict__ dK, int batch, int max_dim, int slots,
-                               FwScratch s) {
+// One thread per matrix (in turns).  The sums of every limit step are formed
+// in one pass: a matrix's candidates are modelled once and picked from
+// kSimtSteps + 1 times.
+__global__ void __launch_bounds__(kPlanThreads)
+    fw_plan_kernel(const int* __restrict__ dM, const int* __restrict__ dN,
+                   const int* __restrict__ dK, int batch, int max_dim, int slots, FwScratch s) {
   __shared__ int bin_tiles[kBins];
   __shared__ int bin_start[kBins];
-  __shared__ unsigned long long work, dwork;
-  __shared__ int changed;
+  __shared__ unsigned long long work[kSimtSteps + 1];
+  __shared__ int longest[kSimtSteps + 1];  // non-negative floats order as ints
+  __shared__ float limit;
   for (int b = threadIdx.x; b < kBins; b += blockDim.x) bin_tiles[b] = 0;
-  if (threadIdx.x == 0) work = 0;
+  if (threadIdx.x <= kSimtSteps) {
+    work[threadIdx.x] = 0;
+    longest[threadIdx.x] = 0;
+  }
   __syncthreads();
-  // per-matrix choice (mat_start: -1 no output, 0 has tiles, until the end)
+  auto sums = [&](int from, int to) {
+    for (int i0 = 0; i0 < batch; i0 += blockDim.x) {
+      const int i = i0 + threadIdx.x;
+      const int M = i < batch ? dM[i] : 0, N = i < batch ? dN[i] : 0, K = i < batch ? dK[i] : 0;
+      const bool any = !fw_bad(M, N, K, max_dim) && M > 0 && N > 0;
+      SimtCands e;
+      if (any) simt_cands(M, N, K, -1, c_cfgs, c_cost, &e);
+      for (int j = from; j <= to; ++j) {
+        float w = 0.0f, l = 0.0f;
+        if (any) {
+          const float T = j == 0 ? 3e38f : simt_limit(__int_as_float(longest[0]), j);
+          if (simt_pick(e, T, &w, &l) < 0) w = l = 0.0f;
+        }
+        long long v = (long long)w;
+        int m = __float_as_int(l);
+        for (int o = 16; o; o >>= 1) {
+          v += __shfl_xor_sync(0xffffffffu, v, o);
+          m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        }
+        if ((threadIdx.x & 31) == 0 && m > 0) {
+          atomicAdd(&work[j], (unsigned long long)v);
+          atomicMax(&longest[j], m);
+        }
+      }
+    }
+    __syncthreads();
+  };
+  sums(0, 0);
+  sums(1, kSimtSteps);
+  if (threadIdx.x == 0) {
+    long long w[kSimtSteps + 1];
+    float l[kSimtSteps + 1];
+    for (int j = 0; j <= kSimtSteps; ++j) {
+      w[j] = (long long)work[j];
+      l[j] = __int_as_float(longest[j]);
+    }
+    limit = simt_choose_limit(w, l, slots);
+  }
+  __syncthreads();
+  // each matrix reserves its tiles in the bin of its tile time
   for (int i = threadIdx.x; i < batch; i += blockDim.x) {
     const int M = dM[i], N = dN[i], K = dK[i];
-    const FwMat r = fw_plan_matrix(M, N, K, max_dim, c_cfgs, c_cost);
-    if (r.bad) atomicOr(s.err, 1);
-    s.descs[i] = MatDesc{M, N, K, max(M, 1), max(K, 1), max(M, 1), r.cfg < 0 ? 0 : r.cfg, 0};
-    s.mat_start[i] = r.cfg < 0 ? -1 : 0;
-    if (r.cfg >= 0) atomicAdd(&work, (unsigned long long)fw_work(M, N, K, r.cfg, c_cfgs, c_cost));
-  }
-  // parallelism rebalance in rounds, each against the round's starting total
-  for (int round = 0; round < kRebalanceRounds; ++round) {
-    __syncthreads();
-    const long long W = (long long)work;
-    if (threadIdx.x == 0) {
-      dwork = 0;
-      changed = 0;
+    MatDesc d{M, N, K, max(M, 1), max(K, 1), max(M, 1), 0, 0};
+    int start = -1;
+    if (fw_bad(M, N, K, max_dim)) {
+      atomicOr(s.err, 1);
+    } else if (M > 0 && N > 0) {
+      SimtCands e;
+      float w, l;
+      simt_cands(M, N, K, -1, c_cfgs, c_cost, &e);
+      const int c = simt_pick(e, limit, &w, &l);
+      if (c >= 0) {
+        d.cfg = c;
+        d.aux = fw_bin(K, c_cost[c]);
+        start = atomicAdd(&bin_tiles[d.aux], (int)simt_tiles(M, N, c_cfgs[c]));
+      }
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < batch; i += blockDim.x) {
-      if (s.mat_start[i] < 0) continue;
-      const MatDesc d = s.descs[i];
-      const int c2 = fw_rebalance(d.M, d.N, d.K, d.cfg, W, slots, c_cfgs, c_cost);
-      if (c2 < 0) continue;
-      atomicAdd(&dwork, (unsigned long long)(fw_work(d.M, d.N, d.K, c2, c_cfgs, c_cost) -
-                                            fw_work(d.M, d.N, d.K, d.cfg, c_cfgs, c_cost)));
-      s.descs[i].cfg = c2;
-      changed = 1;
-    }
-    __syncthreads();
-    if (!changed) break;
-    if (threadIdx.x == 0) work = (unsigned long long)W + dwork;
-  }
-  __syncthreads();
-  // bins of the final tile times; each matrix reserves its tiles in its bin
-  for (int i = threadIdx.x; i < batch; i += blockDim.x) {
-    if (s.mat_start[i] < 0) continue;
-    const MatDesc d = s.descs[i];
-    const int bin = min(kBins - 1, max(0, quarter_octave(fw_tile_ns(d.K, c_cost[d.cfg])) - 24));
-    s.descs[i].aux = bin;
-    s.mat_start[i] = atomicAdd(&bin_tiles[bin], (int)fw_tiles(d.M, d.N, c_cfgs[d.cfg]));
+    s.descs[i] = d;
+    s.mat_start[i] = start;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -202,8 +151,7 @@ __global__ void fw_expand_kernel(int batch, FwScratch s) {
   const int start = s.mat_start[warp];
   if (start < 0) return;
   const MatDesc d = s.descs[warp];
-  const int tmx = (d.M + c_cfgs[d.cfg].bm - 1) / c_cfgs[d.cfg].bm;
-  const int tnx = (d.N + c_cfgs[d.cfg].bn - 1) / c_cfgs[d.cfg].bn;
+  const int tmx = simt_tiles_m(d.M, c_cfgs[d.cfg]), tnx = simt_tiles_n(d.N, c_cfgs[d.cfg]);
   const int tiles = tmx * tnx;
   for (int t = lane; t < tiles; t += 32)
     s.items[start + t] = TileItem{warp, (uint16_t)(t % tmx), (uint16_t)(t / tmx)};
@@ -289,7 +237,7 @@ extern "C" bgemm_status_t bgemm_framework_gemm(const int* dM, const int* dN, con
     ctx.cap_items = ci;
   }
   const int grid = df.num_sms * df.simt_ctas_per_sm;
-  fw_plan_kernel<<<1, 1024, 0, stream>>>(dM, dN, dK, batch, max_dim, grid, ctx.s);
+  fw_plan_kernel<<<1, kPlanThreads, 0, stream>>>(dM, dN, dK, batch, max_dim, grid, ctx.s);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_error(e, "framework plan kernel");
   fw_expand_kernel<<<(batch + 7) / 8, 256, 0, stream>>>(batch, ctx.s);
@@ -344,7 +292,7 @@ cudaError_t fw_launch_on_scratch(const int* dM, const int* dN, const int* dK, fl
       ctx.consts = true;
     }
   }
-  fw_plan_kernel<<<1, 1024, 0, stream>>>(dM, dN, dK, batch, max_dim, grid, s);
+  fw_plan_kernel<<<1, kPlanThreads, 0, stream>>>(dM, dN, dK, batch, max_dim, grid, s);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   fw_expand_kernel<<<(batch + 7) / 8, 256, 0, stream>>>(batch, s);
@@ -404,38 +352,35 @@ extern "C" int bgemm_debug_framework_plan(const int* M, const int* N, const int*
   if (batch < 0 || !err || slots < 1 || (batch > 0 && (!M || !N || !K))) return -1;
   std::vector<int> cfg(batch, -1);
   std::vector<int> start(batch, -1);
-  int bin_tiles[kBins] = {};
-  *err = 0;
-  long long W = 0;
-  for (int i = 0; i < batch; ++i) {
-    const FwMat r = fw_plan_matrix(M[i], N[i], K[i], max_dim, kSimtCfgs, kSimtCost);
-    if (r.bad) *err |= 1;
-    cfg[i] = r.cfg;
-    if (r.cfg >= 0) W += fw_work(M[i], N[i], K[i], r.cfg, kSimtCfgs, kSimtCost);
-  }
-  for (int round = 0; round < kRebalanceRounds; ++round) {
-    long long dW = 0;
-    bool changed = false;
-    for (int i = 0; i < batch; ++i) {
-      if (cfg[i] < 0) continue;
-      const int c2 = fw_rebalance(M[i], N[i], K[i], cfg[i], W, slots, kSimtCfgs, kSimtCost);
-      if (c2 < 0) continue;
-      dW += fw_work(M[i], N[i], K[i], c2, kSimtCfgs, kSimtCost) -
-            fw_work(M[i], N[i], K[i], cfg[i], kSimtCfgs, kSimtCost);
-      cfg[i] = c2;
-      changed = true;
-    }
-    if (!changed) break;
-    W += dW;
-  }
   std::vector<int> bin(batch, 0);
+  std::vector<SimtCands> cand(batch);
+  int bin_tiles[kBins] = {};
+  long long work[kSimtSteps + 1] = {};
+  float longest[kSimtSteps + 1] = {};
+  *err = 0;
+  auto any = [&](int i) { return !fw_bad(M[i], N[i], K[i], max_dim) && M[i] > 0 && N[i] > 0; };
   for (int i = 0; i < batch; ++i) {
+    if (fw_bad(M[i], N[i], K[i], max_dim)) *err |= 1;
+    if (any(i)) simt_cands(M[i], N[i], K[i], -1, kSimtCfgs, kSimtCost, &cand[i]);
+  }
+  for (int j = 0; j <= kSimtSteps; ++j)
+    for (int i = 0; i < batch; ++i) {
+      float w, l;
+      if (!any(i) ||
+          simt_pick(cand[i], j == 0 ? 3e38f : simt_limit(longest[0], j), &w, &l) < 0)
+        continue;
+      work[j] += (long long)w;
+      longest[j] = std::max(longest[j], l);
+    }
+  const float limit = simt_choose_limit(work, longest, slots);
+  for (int i = 0; i < batch; ++i) {
+    float w, l;
+    if (any(i)) cfg[i] = simt_pick(cand[i], limit, &w, &l);
     if (cfg_out) cfg_out[i] = cfg[i];
     if (cfg[i] < 0) continue;
-    bin[i] = std::min(kBins - 1,
-                      std::max(0, quarter_octave(fw_tile_ns(K[i], kSimtCost[cfg[i]])) - 24));
+    bin[i] = fw_bin(K[i], kSimtCost[cfg[i]]);
     start[i] = bin_tiles[bin[i]];
-    bin_tiles[bin[i]] += (int)fw_tiles(M[i], N[i], kSimtCfgs[cfg[i]]);
+    bin_tiles[bin[i]] += (int)simt_tiles(M[i], N[i], kSimtCfgs[cfg[i]]);
   }
   int bin_start[kBins], n = 0;
   for (int b = kBins - 1; b >= 0; --b) {

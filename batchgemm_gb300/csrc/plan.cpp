@@ -91,18 +91,62 @@ bgemm_status_t device_facts(DeviceFacts* out) {
 // ------------------------------------------------------------ planning ----
 static inline long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
 
-// Candidate (cost, tiles) of configuration c for matrix (M, N, K).
-static bool simt_eval(int c, int M, int N, int K, long long* tiles, double* t_tile) {
-  const SimtCfg& g = kSimtCfgs[c];
-  if (ceil_div(M, g.bm) > 65535 || ceil_div(N, g.bn) > 65535) return false;
-  *tiles = ceil_div(M, g.bm) * ceil_div(N, g.bn);
-  *t_tile = kSimtCost[c].a_ns + kSimtCost[c].b_ns * (double)K;
-  return true;
-}
-
+// SIMT tile choice (the model and the rule are in tile_table.h).
 static bgemm_status_t choose_simt(const int* M, const int* N, const int* K, int batch, int slots,
                                   const bgemm_plan_options_t* opt, std::vector<MatPlan>& mp) {
-  return choose_tiles(kSimtNumCfgs, simt_eval, M, N, K, batch, slots, opt, mp);
+  mp.assign(batch, MatPlan{-1, 0, 0.0});
+  const int force = opt ? opt->force_tile_config : -1;
+  std::vector<SimtCands> cand((size_t)batch);
+  std::vector<int> over;              // matrices whose choice the next limit rules out
+  std::vector<float> cur_w, cur_l;    // their work and tile time
+  long long work[kSimtSteps + 1] = {};
+  float longest[kSimtSteps + 1] = {};
+  cur_w.resize((size_t)batch);
+  cur_l.resize((size_t)batch);
+  for (int i = 0; i < batch; ++i) {
+    if (M[i] == 0 || N[i] == 0) continue;
+    simt_cands(M[i], N[i], K[i], force, kSimtCfgs, kSimtCost, &cand[i]);
+    if (simt_pick(cand[i], 3e38f, &cur_w[i], &cur_l[i]) < 0)
+      return set_error(BGEMM_ERROR_NOT_SUPPORTED, 1, i, "matrix %d: no tile configuration fits",
+                       i);
+    over.push_back(i);
+    work[0] += (long long)cur_w[i];
+    longest[0] = std::max(longest[0], cur_l[i]);
+  }
+  float T = 3e38f;
+  if (!(opt && opt->disable_rebalance) && force < 0 &&
+      kSimtTail * longest[0] > 0.02f * ((float)work[0] / (float)slots)) {
+    // a choice stays the least work until its own tile is over the limit, so
+    // each step looks at the matrices above it alone, longest tile first
+    std::sort(over.begin(), over.end(), [&](int a, int b) { return cur_l[a] > cur_l[b]; });
+    for (int j = 1; j <= kSimtSteps; ++j) {
+      const float lim = simt_limit(longest[0], j);
+      work[j] = work[j - 1];
+      size_t n = 0;
+      for (; n < over.size() && cur_l[over[n]] > lim; ++n) {
+        const int i = over[n];
+        work[j] -= (long long)cur_w[i];
+        simt_pick(cand[i], lim, &cur_w[i], &cur_l[i]);
+        work[j] += (long long)cur_w[i];
+      }
+      // (what has no shorter tile stays above every later limit as well)
+      std::sort(over.begin(), over.begin() + n, [&](int a, int b) { return cur_l[a] > cur_l[b]; });
+      std::inplace_merge(over.begin(), over.begin() + n, over.end(),
+                         [&](int a, int b) { return cur_l[a] > cur_l[b]; });
+      longest[j] = over.empty() ? 0.0f : cur_l[over[0]];
+    }
+    T = simt_choose_limit(work, longest, slots);
+  }
+  for (int i = 0; i < batch; ++i) {
+    if (M[i] == 0 || N[i] == 0) continue;
+    float w, l;
+    const int c = simt_pick(cand[i], T, &w, &l);
+    mp[i] = MatPlan{c, simt_tiles(M[i], N[i], kSimtCfgs[c]), simt_tile_ns(K[i], kSimtCost[c])};
+    if (mp[i].tiles > (1LL << 31))
+      return set_error(BGEMM_ERROR_NOT_SUPPORTED, 1, i, "matrix %d: no tile configuration fits",
+                       i);
+  }
+  return BGEMM_SUCCESS;
 }
 
 bgemm_status_t choose_tiles(int ncfg, TileEval eval, const int* M, const int* N, const int* K,
@@ -774,7 +818,8 @@ bgemm_status_t plan_execute(bgemm_plan_t p, float alpha, const float* const* dA,
     SimtParams sp{p->d_descs, p->d_items,  p->n_items, p->d_counters + kHdrItems,
                   p->d_counters, alpha,    beta,       dA, dB, dC};
     if (p->ev_start) cudaEventRecord(p->ev_start, stream);
-    cudaError_t e = simt_launch(sp, p->grid, stream, p->aux_trans != 0);
+    cudaError_t e = simt_launch(sp, p->grid, stream, (p->aux_trans & kTransAFlag) != 0,
+                                (p->aux_trans & kTransBFlag) != 0);
     if (p->ev_stop) cudaEventRecord(p->ev_stop, stream);
     if (e != cudaSuccess) return cuda_error(e, "SIMT launch");
     return BGEMM_SUCCESS;

@@ -10,6 +10,9 @@
 // tile_table_tuned.inc, written by batchgemm_gb300/autotune.py from
 // measurements on the GPU, replaces the defaults below when present.
 #pragma once
+#include <math.h>
+
+#include "bgemm_internal.h"
 
 namespace bgemm {
 
@@ -82,5 +85,108 @@ constexpr unsigned char kTcGroupTable[3][8] = {
 constexpr int kSimtRingCap = 4;
 constexpr int kTcCPrefetchLead = 0;
 #endif
+
+// ------------------------------------------------- SIMT planning model --
+// Shared by the host planner, the device planner and its host replay, which
+// decide alike: single precision with explicit fmaf, work summed as whole
+// nanoseconds.  `cfgs` and `cost` are kSimtCfgs and kSimtCost, or the device's
+// copies of them.
+//
+// For each matrix the configuration with the least work (modelled time on the
+// CTAs) among those whose single tile takes no longer than a limit T, with T
+// chosen for the batch: the makespan is modelled as the average load of a
+// persistent CTA plus the longest tile (kSimtTail of it), and T runs down from
+// the longest tile of the unlimited choice in steps of sqrt(2).
+constexpr float kSimtTail = 1.0f;     // share of the longest tile that is not hidden
+constexpr float kSimtFma = 0.35f;     // time per k that a skipped edge saves
+constexpr int kSimtSteps = 12;
+
+// (bm, bn, gm and gn are powers of two)
+__host__ __device__ inline int simt_tiles_m(int M, SimtCfg g) { return (M + g.bm - 1) >> g.lm; }
+__host__ __device__ inline int simt_tiles_n(int N, SimtCfg g) { return (N + g.bn - 1) >> g.ln; }
+__host__ __device__ inline bool simt_fits(int M, int N, SimtCfg g) {
+  // TileItem holds 16-bit tile coordinates
+  return simt_tiles_m(M, g) <= 65535 && simt_tiles_n(N, g) <= 65535;
+}
+__host__ __device__ inline long long simt_tiles(int M, int N, SimtCfg g) {
+  return (long long)simt_tiles_m(M, g) * simt_tiles_n(N, g);
+}
+// One full tile's share of a CTA's time.
+__host__ __device__ inline float simt_tile_ns(int K, TileCost t) {
+  return fmaf(t.b_ns, (float)K, t.a_ns);
+}
+// The time a tile takes itself, with the SM nearly to itself, as the last ones
+// run (measured on thin matrices of K = 4096: 38, 55, 94, 33 and 30 ns per k
+// for ids 0, 1, 7, 8, 9; the 128 x 128 tile between that and its busy 219 ns).
+__host__ __device__ inline float simt_alone_ns(int K, TileCost t, int c) {
+  const float f = c == 0 ? 4.5f : c < 7 ? 3.0f : c == 7 ? 0.6f : 0.75f;
+  return fmaf(t.b_ns * f, (float)K, t.a_ns * (c < 7 ? 3.0f : f));
+}
+// All tiles of a matrix.  A ragged edge's FMAs are skipped in steps of gm x gn
+// outputs, its copies are not.
+__host__ __device__ inline float simt_work_ns(int M, int N, int K, SimtCfg g, TileCost t) {
+  const float tiles = (float)simt_tiles(M, N, g);
+  const float done = (float)((M + g.gm - 1) & -g.gm) * (float)((N + g.gn - 1) & -g.gn);
+  const float part = done / (tiles * (float)(g.bm * g.bn));
+  return fmaf(t.b_ns * tiles * fmaf(kSimtFma, part, 1.0f - kSimtFma), (float)K, t.a_ns * tiles);
+}
+// The candidates of one matrix (M, N > 0); lat < 0: not one.
+struct SimtCands {
+  float work[kSimtNumCfgs], lat[kSimtNumCfgs];
+};
+__host__ __device__ inline void simt_cands(int M, int N, int K, int force, const SimtCfg* cfgs,
+                                           const TileCost* cost, SimtCands* e) {
+#pragma unroll
+  for (int c = 0; c < kSimtNumCfgs; ++c) {
+    e->work[c] = 0.0f;
+    e->lat[c] = -1.0f;
+    if ((force >= 0 ? c != force : !simt_auto_cfg(c, M, N)) || !simt_fits(M, N, cfgs[c])) continue;
+    e->work[c] = simt_work_ns(M, N, K, cfgs[c], cost[c]);
+    e->lat[c] = simt_alone_ns(K, cost[c], c);
+  }
+}
+// Least work with a tile of at most T, or else the shortest tile (-1: none).
+__host__ __device__ inline int simt_pick(const SimtCands& e, float T, float* work, float* lat) {
+  int best = -1, any = -1;
+  float bw = 0.0f, bl = 0.0f, sl = 0.0f, sw = 0.0f;
+#pragma unroll
+  for (int c = kSimtNumCfgs - 1; c >= 0; --c) {
+    if (e.lat[c] < 0.0f) continue;
+    if (any < 0 || e.lat[c] < sl) {
+      any = c;
+      sl = e.lat[c];
+      sw = e.work[c];
+    }
+    if (e.lat[c] <= T && (best < 0 || e.work[c] < bw)) {
+      best = c;
+      bw = e.work[c];
+      bl = e.lat[c];
+    }
+  }
+  *work = best >= 0 ? bw : sw;
+  *lat = best >= 0 ? bl : sl;
+  return best >= 0 ? best : any;
+}
+// T from the sums of every step (step 0: no limit; step j: the limit
+// simt_limit(longest[0], j)).
+__host__ __device__ inline float simt_limit(float longest, int step) {
+  float t = longest;
+  for (int j = 0; j < step; ++j) t *= 0.70710678f;
+  return t;
+}
+__host__ __device__ inline float simt_choose_limit(const long long* work, const float* longest,
+                                                   int slots) {
+  float best = 0.0f;
+  int at = 0;
+  for (int j = 0; j <= kSimtSteps; ++j) {
+    if (j > 0 && kSimtTail * simt_limit(longest[0], j - 1) <= 0.02f * best) break;
+    const float m = fmaf(kSimtTail, longest[j], (float)work[j] / (float)slots);
+    if (j == 0 || m < best) {
+      best = m;
+      at = j;
+    }
+  }
+  return at == 0 ? 3e38f : simt_limit(longest[0], at);
+}
 
 }  // namespace bgemm
