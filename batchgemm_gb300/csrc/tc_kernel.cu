@@ -42,6 +42,7 @@
 
 #include "tc_epilogue.h"
 #include "tc_ptx.h"
+#include "tc_split.h"
 
 namespace bgemm {
 namespace {
@@ -72,53 +73,6 @@ constexpr int kGroupKB = 2;
 constexpr int kEpiWarps = 8;
 constexpr int kEpiCols = kTcMaxBN / 2;
 
-// ---------------------------------------------------- operand splitting --
-__device__ __forceinline__ void put(char* hi, char* lo, long long idx, float x, int kind,
-                                    int split) {
-  if (kind == kKindTF32) {
-    const float h = round_keep(x, 13);
-    reinterpret_cast<float*>(hi)[idx] = h;
-    if (split) {
-      const bool fin = (__float_as_uint(x) & 0x7f800000u) != 0x7f800000u;
-      reinterpret_cast<float*>(lo)[idx] = fin ? round_keep(x - h, 13) : 0.0f;
-    }
-  } else {
-    const float h = round_keep(x, 16);
-    reinterpret_cast<uint16_t*>(hi)[idx] = (uint16_t)(__float_as_uint(h) >> 16);
-    if (split) {
-      const bool fin = (__float_as_uint(x) & 0x7f800000u) != 0x7f800000u;
-      const float l = fin ? round_keep(x - h, 16) : 0.0f;
-      reinterpret_cast<uint16_t*>(lo)[idx] = (uint16_t)(__float_as_uint(l) >> 16);
-    }
-  }
-}
-
-// Splits four consecutive k of one packed row and stores hi (and lo) with one
-// 16-byte (TF32) or 8-byte (BF16) store each; idx is a multiple of 4.
-__device__ __forceinline__ void put4(char* hi, char* lo, long long idx, const float* x, int kind,
-                                     int split) {
-  float h[4], l[4];
-  const int drop = (kind == kKindTF32) ? 13 : 16;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    h[i] = round_keep(x[i], drop);
-    const bool fin = (__float_as_uint(x[i]) & 0x7f800000u) != 0x7f800000u;
-    l[i] = fin ? round_keep(x[i] - h[i], drop) : 0.0f;
-  }
-  if (kind == kKindTF32) {
-    *reinterpret_cast<float4*>(reinterpret_cast<float*>(hi) + idx) = make_float4(h[0], h[1], h[2], h[3]);
-    if (split)
-      *reinterpret_cast<float4*>(reinterpret_cast<float*>(lo) + idx) = make_float4(l[0], l[1], l[2], l[3]);
-  } else {
-    auto pk = [](float a, float b) {
-      return (__float_as_uint(a) >> 16) | (__float_as_uint(b) & 0xFFFF0000u);
-    };
-    *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(hi) + idx) = make_uint2(pk(h[0], h[1]), pk(h[2], h[3]));
-    if (split)
-      *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(lo) + idx) = make_uint2(pk(l[0], l[1]), pk(l[2], l[3]));
-  }
-}
-
 // k per chunk of the pre-pass: each thread keeps kPackK / 8 loads in flight.
 constexpr int kPackK = 256;
 
@@ -126,6 +80,7 @@ constexpr int kPackK = 256;
 // thread issues all kPackK / 8 of its loads for a chunk before it stores, and
 // writes four consecutive k per store (rows are 16-byte aligned, so packed
 // writes are full vectors; the K tail and rows past M/N are masked).
+template <int KIND, int SPLIT>
 __global__ void __launch_bounds__(256) tc_pack_kernel(const TcPackParams p) {
   __shared__ float t[kPackK][33];
   const int tid = threadIdx.x;
@@ -172,10 +127,10 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(const TcPackParams p) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) x[i] = t[kk + i][wm];
             if (k + 4 <= K) {
-              put4(hi, lo, mr * kpad + k, x, p.kind, p.split);
+              put4<KIND, SPLIT>(hi, lo, mr * kpad + k, x);
             } else {
               for (int i = 0; i < 4 && k + i < K; ++i)
-                put(hi, lo, mr * kpad + k + i, x[i], p.kind, p.split);
+                put<KIND, SPLIT>(hi, lo, mr * kpad + k + i, x[i]);
             }
           }
         }
@@ -205,7 +160,7 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(const TcPackParams p) {
           for (int h = 0; h < kPackK / 32; ++h) {
             const int k = k0 + 32 * h + lane;
             if (r_w + rr < rows && k < K)
-              put(hi, lo, (long long)(r_w + rr) * kpad + k, x[rr][h], p.kind, p.split);
+              put<KIND, SPLIT>(hi, lo, (long long)(r_w + rr) * kpad + k, x[rr][h]);
           }
         }
       }
@@ -234,10 +189,10 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(const TcPackParams p) {
         for (int h2 = 0; h2 < kPackK / 32; ++h2) {
           const int k = k0 + wk + 32 * h2;
           if (k + 4 <= K) {
-            put4(hi, lo, n * kpad + k, x[h2], p.kind, p.split);
+            put4<KIND, SPLIT>(hi, lo, n * kpad + k, x[h2]);
           } else {
             for (int i = 0; i < 4 && k + i < K; ++i)
-              put(hi, lo, n * kpad + k + i, x[h2][i], p.kind, p.split);
+              put<KIND, SPLIT>(hi, lo, n * kpad + k + i, x[h2][i]);
           }
         }
       }
@@ -651,7 +606,12 @@ cudaError_t tc_tmap_launch(const TcTmapParams& p, cudaStream_t s) {
 
 cudaError_t tc_pack_launch(const TcPackParams& p, int grid, cudaStream_t s) {
   if (p.n_jobs == 0 && !p.n_jobs_dev) return cudaSuccess;
-  tc_pack_kernel<<<grid, 256, 0, s>>>(p);
+  if (p.kind == kKindBF16)
+    tc_pack_kernel<kKindBF16, 1><<<grid, 256, 0, s>>>(p);
+  else if (p.split)
+    tc_pack_kernel<kKindTF32, 1><<<grid, 256, 0, s>>>(p);
+  else
+    tc_pack_kernel<kKindTF32, 0><<<grid, 256, 0, s>>>(p);
   return cudaGetLastError();
 }
 

@@ -56,16 +56,6 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t a, uint32_t parit
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
-// Round to nearest, ties to even, keeping 23 - drop explicit mantissa bits
-// (TF32: drop 13, BF16: drop 16); Inf and NaN pass through.
-__device__ __forceinline__ float round_keep(float x, int drop) {
-  uint32_t u = __float_as_uint(x);
-  if ((u & 0x7f800000u) == 0x7f800000u) return x;
-  const uint32_t half = (1u << (drop - 1)) - 1u;
-  u += half + ((u >> drop) & 1u);
-  u &= ~((1u << drop) - 1u);
-  return __uint_as_float(u);
-}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1,
                                             uint32_t bar) {
   asm volatile(
