@@ -474,6 +474,7 @@ static bgemm_status_t plan_commit(bgemm_plan_s* p, BatchPlan& bp, bool first,
   int* hdr = reinterpret_cast<int*>(h);
   hdr[kHdrItems] = bp.req.tiles;
   hdr[kHdrJobs] = bp.req.pack_jobs;
+  if (p->tc) hdr[kHdrHead] = tc_head_jobs(p);
   if (bp.batch) std::memcpy(h + p->off_descs, bp.descs.data(), sizeof(MatDesc) * bp.descs.size());
   if (!bp.items.empty())
     std::memcpy(h + p->off_items, bp.items.data(), sizeof(TileItem) * bp.items.size());

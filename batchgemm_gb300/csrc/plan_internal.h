@@ -29,13 +29,15 @@ constexpr int kTcSwapFlag = 1 << 30;
 // ids 0..7: one-SM tiles; ids 8..15: CTA-pair tiles (split modes)
 constexpr int kTcNumCfgs = 16;
 
-// The plan's device header (256 bytes, ints): [0] queue head and [1] CTAs
-// finished (reset by the kernels themselves), [kHdrItems] work items of the
-// current batch, [kHdrJobs] pre-pass jobs of the current batch.  Kernels read
+// The plan's device header (256 bytes, ints): [0] queue head, [1] CTAs
+// finished and [2] head of the GEMM kernel's own packing queue (reset by the
+// kernels themselves), [kHdrItems] work items of the current batch, [kHdrJobs]
+// its packing jobs, [kHdrHead] those of them that the pre-pass kernel does.  Kernels read
 // the counts from here, so a captured launch serves every batch an update
 // uploads.
 constexpr int kHdrItems = 16;
 constexpr int kHdrJobs = 17;
+constexpr int kHdrHead = 18;
 constexpr size_t kHdrBytes = 256;
 // Pinned staging buffers of a plan's uploads, used in turn: an update waits
 // only for the upload kStageBufs updates back to have been consumed.
@@ -121,6 +123,8 @@ void tc_tile_dims(bgemm_plan_s* p, int i, int M, int N, int cfg, int* bm, int* b
 void tc_layout(bgemm_plan_s* p, const std::vector<MatDesc>& hd, bgemm_plan_requirements_t* req);
 // tc_alloc: device/pinned buffers for the plan's capacity, launch shapes.
 bgemm_status_t tc_alloc(bgemm_plan_s* p);
+// packing jobs of the laid-out batch that the pre-pass kernel does
+int tc_head_jobs(const bgemm_plan_s* p);
 // tc_commit: stage and upload the laid-out batch through staging buffer
 // `stage`, build its tensor maps (first: also templates and error word).
 bgemm_status_t tc_commit(bgemm_plan_s* p, int stage, int batch, bool first, cudaStream_t stream);

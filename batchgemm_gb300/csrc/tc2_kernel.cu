@@ -41,6 +41,7 @@
 
 #include "tc_epilogue.h"
 #include "tc_ptx.h"
+#include "tc_split.h"
 #include "tile_table.h"
 
 namespace bgemm {
@@ -51,6 +52,12 @@ constexpr int kA = kRows * 128;            // 16 KB per part
 constexpr int kB = 128 * 128;              // B-side half: up to 128 rows
 constexpr int kNAcc = 2;                   // 256-column accumulator buffers
 constexpr int kSched = 4;                  // schedule slots (items published ahead)
+// Packing warps (warps 2 and 3, otherwise idle): each loads a strip of 32 packed rows in chunks
+// of 32 k through a ring of four buffers, [k][33] floats where rows are
+// contiguous in memory and [row][32] where k is.
+constexpr int kPackWarps = 2, kPackBufs = 4, kPackK2 = 32;
+constexpr int kPackFloats = kPackK2 * 33;
+constexpr int kPackBytes = kPackFloats * 4;
 // Stage ring of 3 stages of 64 KB, two parts per side: the split modes' hi and
 // lo halves of one 128-byte K slice, or two consecutive K slices of the
 // single-product TF32 mode (four TMA boxes per stage either way: one thread
@@ -61,14 +68,16 @@ struct Geo2 {
   static constexpr int STAGE = NP * (kA + kB);
   static constexpr int S = 3;
   static constexpr int NBAR = 2 * S + 2 * kNAcc + 1 + 2 * kSched;
-  // barriers | TMEM address, abort flag (16 B) | schedule slots | alignment
-  static constexpr int SMEM = S * STAGE + NBAR * 8 + 16 + 4 * kSched + 1024;
+  // barriers | TMEM address, abort flag (16 B) | schedule slots | packing
+  // warps' buffers (16-byte aligned) | alignment of the whole
+  static constexpr int PACK = (S * STAGE + NBAR * 8 + 16 + 4 * kSched + 15) / 16 * 16;
+  static constexpr int SMEM = PACK + kPackWarps * kPackBufs * kPackBytes + 1024;
 };
 constexpr int kSmemMax = Geo2<1>::SMEM > Geo2<0>::SMEM ? Geo2<1>::SMEM : Geo2<0>::SMEM;
 constexpr int kEpiWarps2 = 8;              // 2 per TMEM lane quadrant
 constexpr int kCols = 128;                 // accumulator columns per epilogue warp
 // Three warpgroups: warpgroup 0 = producer (warp 0), MMA issuer (warp 1) and
-// two idle warps; warpgroups 1 and 2 = the 8 epilogue warps.  At launch every
+// two packing warps; warpgroups 1 and 2 = the 8 epilogue warps.  At launch every
 // thread gets 168 registers (3 warps per SM sub-partition); warpgroup 0 gives
 // most of its share to the epilogue warps, whose 128 accumulator columns per
 // lane would otherwise spill: 128 x 56 + 256 x 224 = 384 x 168.
@@ -101,6 +110,188 @@ __device__ __forceinline__ uint32_t make_idesc_pair(int n) {
   constexpr uint32_t fmt = (KIND == kKindTF32) ? 2u : 1u;
   return (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(n >> 3) << 17) |
          ((uint32_t)(256 >> 4) << 24);
+}
+
+__device__ __forceinline__ void cp4(uint32_t dst, const float* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void cp16(uint32_t dst, const float* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes)
+               : "memory");
+}
+
+// A packing warp: pulls strips behind the pre-pass kernel's and splits them as
+// tc_pack_kernel does, three chunks on their way while one is written.  A
+// finished strip is published by a release on its matrix's count, behind a
+// proxy fence: the readers are TMA loads.
+// Bound by the issue of one warp: alone on the chip the 304 of them split the
+// skewed batch's 5.5 GB of operands in 3.5 ms (4.2 ms before inner chunks lost
+// their bounds), beside the GEMM in 5.7.  The copies also cost the GEMM: they
+// fill shared memory by 32-byte wavefronts beside the MMAs' operand reads.
+// Skewed batch, pre-pass then GEMM 9.45 ms, this way 8.6 to 9.0; a limit on how
+// far packing runs ahead of the tiles (one to eight waves) changed nothing.
+template <int KIND, int SPLIT>
+__device__ __forceinline__ void pack_strips(const TcGemmParams& p, float* buf, int lane,
+                                            volatile int* abort) {
+  const int n_jobs = *p.n_jobs, n_head = *p.n_head;
+  if (n_head >= n_jobs) return;
+#pragma unroll 1
+  for (;;) {
+    int j = 0;
+    if (lane == 0) j = *abort ? n_jobs : n_head + atomicAdd(p.counters + 2, 1);
+    j = __shfl_sync(0xffffffffu, j, 0);
+    if (j >= n_jobs) return;
+    const PackJob job = p.jobs[j];
+    const bool is_a = job.op == 0;
+    int K, rows, ld;
+    bool rows_contig;
+    {
+      const MatDesc d = p.descs[job.mat];
+      K = d.K;
+      rows = (is_a ? d.M : d.N) - job.r0;
+      ld = is_a ? d.lda : d.ldb;
+      rows_contig = is_a ? !(d.aux & kTransAFlag) : (d.aux & kTransBFlag) != 0;
+    }
+    const float* X = is_a ? p.A[job.mat] : p.B[job.mat];
+    X += rows_contig ? (long long)job.r0 : (long long)job.r0 * ld;
+    const bool vec = ((reinterpret_cast<uintptr_t>(X) & 15u) == 0) && (ld & 3) == 0;
+    // one chunk's copies; inner ones carry no bounds
+    auto load = [&](int k0, float* s) {
+      const uint32_t dst = smem_u32(s) + lane * 4;
+      const int ks = K - k0;
+      if (rows_contig) {
+        const float* src = X + (long long)k0 * ld + lane;
+        const int bytes = lane < rows ? 4 : 0;
+        if (ks >= kPackK2) {
+#pragma unroll
+          for (int k = 0; k < kPackK2; ++k) cp4(dst + k * 132, src + (long long)ld * k, bytes);
+        } else {
+#pragma unroll 4
+          for (int k = 0; k < kPackK2; ++k)
+            cp4(dst + k * 132, src + (long long)ld * k, k < ks ? bytes : 0);
+        }
+      } else if (vec) {
+        const int kq = (lane & 7) * 4, r0 = lane >> 3;
+        const int bytes = min(max(ks - kq, 0), 4) * 4;
+        const float* src = X + (long long)r0 * ld + k0 + kq;
+#pragma unroll
+        for (int r = 0; r < 32; r += 4)
+          cp16(smem_u32(s) + ((r0 + r) * kPackK2 + kq) * 4, src + (long long)ld * r,
+               r0 + r < rows ? bytes : 0);
+      } else {
+        const float* src = X + k0 + lane;
+        const int bytes = lane < ks ? 4 : 0;
+        if (rows >= 32) {
+#pragma unroll
+          for (int r = 0; r < 32; ++r) cp4(dst + r * 128, src + (long long)ld * r, bytes);
+        } else {
+#pragma unroll 4
+          for (int r = 0; r < 32; ++r)
+            cp4(dst + r * 128, src + (long long)ld * r, r < rows ? bytes : 0);
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const PackDesc* pd = p.pdescs + job.mat;
+    const int kpad = pd->kpad;
+    constexpr int E = KIND == kKindTF32 ? 4 : 2;  // bytes of a packed element
+    // eight lanes to a packed row, four k each; four rows at a time
+    const int r4 = lane >> 3, kq = (lane & 7) * 4;
+    const long long at0 = (long long)(job.r0 + r4) * kpad + kq;
+    char* hi = p.ws + (is_a ? pd->a_hi : pd->b_hi) + at0 * E;
+    char* lo = p.ws + (is_a ? pd->a_lo : pd->b_lo) + at0 * E;
+    const long long step = 4ll * kpad;  // elements
+#pragma unroll 1
+    for (int c = 0; c < kPackBufs - 1; ++c) {
+      if (c * kPackK2 < K)
+        load(c * kPackK2, buf + c * kPackFloats);
+      else
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    int rd = 0, wr = kPackBufs - 1;
+#pragma unroll 1
+    for (int k0 = 0; k0 < K; k0 += kPackK2) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kPackBufs - 2) : "memory");
+      __syncwarp();  // (and every lane is done with the buffer that is filled next)
+      if (k0 + (kPackBufs - 1) * kPackK2 < K)
+        load(k0 + (kPackBufs - 1) * kPackK2, buf + wr * kPackFloats);
+      else
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      const float* s = buf + rd * kPackFloats + (rows_contig ? kq * 33 + r4 : r4 * kPackK2 + kq);
+      auto fetch = [&](int it, float(&x)[4]) {
+        if (rows_contig) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) x[i] = s[i * 33 + it * 4];
+        } else {
+          const float4 v = *reinterpret_cast<const float4*>(s + it * 4 * kPackK2);
+          x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+        }
+      };
+      if (rows >= 32 && k0 + kPackK2 <= K) {
+        // (four rows of fragments at a time, for their latencies to overlap)
+#pragma unroll
+        for (int i0 = 0; i0 < 8; i0 += 4) {
+          float x[4][4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) fetch(i0 + i, x[i]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) put4<KIND, SPLIT>(hi, lo, (i0 + i) * step, x[i]);
+        }
+      } else {
+#pragma unroll 1
+        for (int it = 0; it < 8; ++it) {
+          const int left = K - k0 - kq;
+          if (it * 4 + r4 < rows && left > 0) {
+            float x[4];
+            fetch(it, x);
+            if (left >= 4) {
+              put4<KIND, SPLIT>(hi, lo, it * step, x);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 3; ++i)
+                if (i < left) put<KIND, SPLIT>(hi, lo, it * step + i, x[i]);
+            }
+          }
+        }
+      }
+      hi += kPackK2 * E;
+      lo += kPackK2 * E;
+      rd = rd + 1 == kPackBufs ? 0 : rd + 1;
+      wr = wr + 1 == kPackBufs ? 0 : wr + 1;
+    }
+    __syncwarp();
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __threadfence();
+    asm volatile("fence.proxy.async.global;" ::: "memory");
+    __syncwarp();
+    if (lane == 0)
+      asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(p.ready + job.mat) : "memory");
+  }
+}
+
+// Waits (bounded) until `need` strips of a matrix are packed.
+__device__ __forceinline__ bool wait_packed(const int* ready, int need, int* err,
+                                            volatile int* abort, unsigned long long limit_ns) {
+  auto done = [&]() {
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(ready) : "memory");
+    return v >= need;
+  };
+  if (!done()) {
+    const uint64_t t0 = gtimer();
+    while (!done()) {
+      __nanosleep(100);
+      if (*abort) return false;
+      if (gtimer() - t0 > limit_ns) {
+        atomicOr(err, 1);
+        *abort = 1;
+        return false;
+      }
+    }
+  }
+  asm volatile("fence.proxy.async.global;" ::: "memory");
+  return true;
 }
 
 // BETA: the launch's beta is nonzero (C is read: late L2 prefetch, 16 reads in
@@ -232,7 +423,13 @@ __global__ void __launch_bounds__(kThreads2, 1) tc2_gemm_kernel(const TcGemmPara
           const int hb = bn >> 1;
           const CUtensorMap* tm = p.tmaps + 4 * ti.mat;
           if (ti.mat != last_mat && d.K > 0) {
+            const int await = p.jobs ? p.pdescs[ti.mat].await : 0;
             for (int q = 0; q < 4; ++q) tmap_acquire(tm + q);
+            if (await > 0 &&
+                !wait_packed(p.ready + ti.mat, await, p.error, abort, p.timeout_ns)) {
+              ok = false;
+              break;
+            }
             last_mat = ti.mat;
           }
           const int nk = (d.K + KE - 1) / KE;           // 128-byte K slices
@@ -406,7 +603,12 @@ __global__ void __launch_bounds__(kThreads2, 1) tc2_gemm_kernel(const TcGemmPara
         wait_bounded(drain, 0, p.error, nullptr, p.timeout_ns);
       }
       __syncwarp();
-    }  // warps 2 and 3 are idle
+    } else if (p.jobs) {
+      // ------------------------------------------- packing (both CTAs)
+      pack_strips<KIND, SPLIT>(
+          p, reinterpret_cast<float*>(smem + G::PACK + (warp - 2) * kPackBufs * kPackBytes), lane,
+          abort);
+    }
   } else {
     // -------------------------------------------- epilogue (both CTAs)
     regs_grow<kRegsEpi>();
@@ -512,15 +714,26 @@ __global__ void __launch_bounds__(kThreads2, 1) tc2_gemm_kernel(const TcGemmPara
   cluster_sync();
   tc_fence_after();
   if (warp == 1) tmem_dealloc_pair(tmem, 512);
-  if (leader && threadIdx.x == 0) {
-    // the last cluster to finish resets the queue for the next launch (every
-    // leader has pulled its final item before it gets here)
-    __threadfence();
-    const unsigned prev = atomicAdd(reinterpret_cast<unsigned*>(p.counters) + 1, 1u);
-    if (prev == (unsigned)ncl - 1) {
-      atomicExch(p.counters, 0);
-      atomicExch(p.counters + 1, 0);
+  if (leader) {
+    // the last cluster to finish resets the queues for the next launch (every
+    // leader has pulled its final item, and every packing warp published its
+    // last strip, before it gets here)
+    if (threadIdx.x == 0) {
       __threadfence();
+      const unsigned prev = atomicAdd(reinterpret_cast<unsigned*>(p.counters) + 1, 1u);
+      const bool last = prev == (unsigned)ncl - 1;
+      if (last) {
+        atomicExch(p.counters, 0);
+        atomicExch(p.counters + 1, 0);
+        atomicExch(p.counters + 2, 0);
+        __threadfence();
+      }
+      slots[0] = last ? 1 : 0;
+    }
+    if (p.jobs && *p.n_head < *p.n_jobs) {
+      __syncthreads();
+      if (slots[0])
+        for (int i = threadIdx.x; i < p.n_ready; i += kThreads2) p.ready[i] = 0;
     }
   }
   if (p.cta_times && threadIdx.x == 0) p.cta_times[2 * blockIdx.x + 1] = gtimer();

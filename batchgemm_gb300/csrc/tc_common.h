@@ -64,7 +64,8 @@ struct PackJob {
 struct PackDesc {
   long long a_hi, a_lo, b_hi, b_lo;
   int kpad;  // row length in elements (K rounded up to 16 bytes)
-  int pad[3];
+  int await; // strips that the GEMM kernel packs itself (0: the pre-pass did)
+  int pad[2];
 };
 
 struct TcPackParams {
@@ -93,6 +94,18 @@ struct TcGemmParams {
   unsigned long long timeout_ns;
   unsigned long long* cta_times;  // if set: [2 * blockIdx] start, [+1] end (global timer, ns)
   TcSchedule sched;               // promotion groups of the split modes (pair kernel)
+  // Pair kernel: pre-pass strips that its idle warps pack while the tensor
+  // cores work (jobs *n_head .. *n_jobs - 1); counters[2] is their queue head,
+  // ready[i] the finished ones of matrix i.  jobs null: there are none.
+  const PackDesc* pdescs;
+  const PackJob* jobs;
+  const int* n_head;
+  const int* n_jobs;
+  int* ready;
+  int n_ready;
+  char* ws;
+  const float* const* A;
+  const float* const* B;
 };
 // The schedule the kernels use for a mode: the autotuned table, or a process-
 // wide override set through bgemm_debug_set_tc_schedule (the autotuner's sweep).

@@ -16,6 +16,7 @@
 namespace bgemm {
 
 struct TcPlan {
+  int mode = BGEMM_MODE_TF32X3;
   int kind = kKindTF32;
   int split = 1;             // the kernels read hi/lo pairs (kind TF32/BF16 split modes)
   bool split_mode = true;    // the plan's mode is TF32X3 or BF16X3
@@ -29,17 +30,19 @@ struct TcPlan {
   void* d_ws = nullptr;      // split operands
   void* d_mem = nullptr;     // templates | tensor maps | pack descs | jobs | error word
   void* h_stage[kStageBufs] = {};  // pinned staging ring, same layout as d_mem
-  size_t off_tm = 0, off_pd = 0, off_jobs = 0, off_err = 0, mem_bytes = 0;
+  size_t off_tm = 0, off_pd = 0, off_jobs = 0, off_err = 0, off_ready = 0, mem_bytes = 0;
   CUtensorMap* d_templ = nullptr;
   CUtensorMap* d_tmaps = nullptr;
   PackDesc* d_pdescs = nullptr;
   PackJob* d_jobs = nullptr;
   int* d_err = nullptr;
+  int* d_ready = nullptr;    // finished strips per matrix (reset by the GEMM kernel)
   int n_jobs = 0;
   int pack_grid = 1;
   // layout of the last planned batch, uploaded by tc_commit
   std::vector<PackDesc> pd;
   std::vector<PackJob> jobs;
+  int head = 0;              // jobs of the pre-pass kernel; the GEMM kernel does the rest
 };
 
 static inline long long cdiv(long long a, long long b) { return (a + b - 1) / b; }
@@ -88,6 +91,7 @@ static bool tc_eval(int c, int M, int N, int K, long long* tiles, double* t_tile
 bgemm_status_t tc_init(bgemm_plan_s* p, const bgemm_plan_options_t* opt, int clusters) {
   auto* t = new TcPlan();
   p->tc = t;
+  t->mode = p->mode;
   t->kind = (p->mode == BGEMM_MODE_BF16X3) ? kKindBF16 : kKindTF32;
   t->split_mode = p->mode != BGEMM_MODE_TF32;
   t->split = t->split_mode ? 1 : 0;
@@ -162,6 +166,50 @@ void tc_tile_dims(bgemm_plan_s* p, int, int, int, int cfg, int* bm, int* bn, Mat
   d->aux = (d->aux & ~kTcSwapFlag) | (tc_cfg_swap(cfg) ? kTcSwapFlag : 0);
 }
 
+int tc_head_jobs(const bgemm_plan_s* p) { return p->tc->head; }
+
+// Tiles of a matrix in its configuration.
+static long long tc_tiles(const MatDesc& d, bool pair) {
+  const bool swap = tc_cfg_swap(d.cfg);
+  const int bm = pair ? 256 : kTcBM, bn = pair ? tc2_cfg_bn(d.cfg) : tc_cfg_bn(d.cfg);
+  return cdiv(swap ? d.N : d.M, bm) * cdiv(swap ? d.M : d.N, bn);
+}
+// The division of the packing between the pre-pass kernel (the first matrices
+// of the job order) and the pair kernel's idle warps (the rest): the shortest
+// head that gives every CTA pair kHeadTiles tiles to start with and keeps each
+// later matrix's packing, at kFuseBytesPerNs of raw operands, ahead of the
+// modelled time at which its tiles begin.  Returns the number of jobs.
+// Measured: 2, 4 and 8 tiles per pair 6.81, 6.83 and 6.88 ms (a stream of four
+// batches) and 538, 525 and 534 us (96 matrices in 3xBF16); 800, 1200 and 2000
+// bytes per ns 1283, 1230 and 1235 us (128 matrices in TF32, whose GEMM is the
+// shortest beside its packing).
+constexpr int kHeadTiles = 4;
+constexpr double kFuseBytesPerNs = 1200.0;
+static int tc_divide(TcPlan* t, const std::vector<MatDesc>& hd, const std::vector<int>& order) {
+  if (!t->pair) return (int)t->jobs.size();
+  // packing done and GEMM begun, in ns from the GEMM kernel's start, if all
+  // the packing were fused
+  double pack = 0, gemm = 0, late = 0;
+  for (int i : order) {
+    const MatDesc& d = hd[i];
+    const TileCost c = kTcCost[t->mode - 1][d.cfg];
+    pack += 4.0 * ((double)d.M + d.N) * d.K / kFuseBytesPerNs;
+    late = std::max(late, pack - gemm);
+    gemm += (double)tc_tiles(d, true) * (c.a_ns + c.b_ns * d.K) / t->clusters;
+  }
+  long long tiles = 0;
+  int jobs = 0;
+  pack = 0;
+  for (int i : order) {
+    const MatDesc& d = hd[i];
+    if (tiles >= (long long)kHeadTiles * t->clusters && pack >= late) break;
+    pack += 4.0 * ((double)d.M + d.N) * d.K / kFuseBytesPerNs;
+    tiles += tc_tiles(d, true);
+    jobs += (int)(cdiv(d.M, 32) + cdiv(d.N, 32));
+  }
+  return jobs;
+}
+
 // Workspace: per matrix [A hi][A lo][B hi][B lo], rows of kpad elements;
 // pack jobs: strips of 32 rows, matrices with the longest K first.
 void tc_layout(bgemm_plan_s* p, const std::vector<MatDesc>& hd, bgemm_plan_requirements_t* req) {
@@ -195,6 +243,8 @@ void tc_layout(bgemm_plan_s* p, const std::vector<MatDesc>& hd, bgemm_plan_requi
     for (int r = 0; r < hd[i].M; r += 32) t->jobs.push_back(PackJob{i, 0, r, 0});
     for (int r = 0; r < hd[i].N; r += 32) t->jobs.push_back(PackJob{i, 1, r, 0});
   }
+  t->head = tc_divide(t, hd, order);
+  for (size_t j = (size_t)t->head; j < t->jobs.size(); ++j) t->pd[t->jobs[j].mat].await++;
   req->pack_jobs = (int)std::min<size_t>(t->jobs.size(), (size_t)1 << 30);
   req->workspace_bytes = std::max<size_t>(off, 256);
   req->kernel_family = t->pair ? 2 : 1;
@@ -274,7 +324,8 @@ bgemm_status_t tc_alloc(bgemm_plan_s* p) {
   t->off_pd = t->off_tm + sizeof(CUtensorMap) * 4 * (size_t)t->cap_batch;
   t->off_jobs = t->off_pd + align256(sizeof(PackDesc) * (size_t)t->cap_batch);
   t->off_err = t->off_jobs + align256(sizeof(PackJob) * (size_t)t->cap_jobs);
-  t->mem_bytes = t->off_err + 256;
+  t->off_ready = t->off_err + 256;
+  t->mem_bytes = t->off_ready + align256(sizeof(int) * (size_t)t->cap_batch);
 
   cudaError_t e = cudaMalloc(&t->d_ws, t->cap_ws);
   if (e != cudaSuccess)
@@ -295,6 +346,7 @@ bgemm_status_t tc_alloc(bgemm_plan_s* p) {
   t->d_pdescs = reinterpret_cast<PackDesc*>(dm + t->off_pd);
   t->d_jobs = reinterpret_cast<PackJob*>(dm + t->off_jobs);
   t->d_err = reinterpret_cast<int*>(dm + t->off_err);
+  t->d_ready = reinterpret_cast<int*>(dm + t->off_ready);
   // 16 CTAs per SM, ~5 waves of the 3 that fit: a shorter last wave than 8 per
   // SM (measured: the skewed pre-pass 3.03 -> 2.98 ms; 4 per SM, 1.3 waves, 3.63)
   t->pack_grid = (int)std::max<long long>(
@@ -336,7 +388,8 @@ bgemm_status_t tc_commit(bgemm_plan_s* p, int stage, int batch, bool first, cuda
   cudaError_t e = cudaSuccess;
   if (first) {
     e = copy(0, t->off_tm);  // templates
-    if (e == cudaSuccess) e = copy(t->off_err, 256);  // zero error word
+    // zero error word and strip counts
+    if (e == cudaSuccess) e = copy(t->off_err, t->mem_bytes - t->off_err);
   }
   if (e == cudaSuccess && t->host_tmaps) e = copy(t->off_tm, sizeof(CUtensorMap) * 4 * (size_t)batch);
   if (e == cudaSuccess) e = copy(t->off_pd, sizeof(PackDesc) * (size_t)batch);
@@ -396,14 +449,17 @@ bgemm_status_t tc_execute(bgemm_plan_s* p, float alpha, const float* const* dA,
                           const float* const* dB, float beta, float* const* dC,
                           cudaStream_t stream) {
   TcPlan* t = p->tc;
-  TcPackParams pp{p->d_descs, t->d_pdescs,  t->d_jobs, t->n_jobs, p->d_counters + kHdrJobs,
+  TcPackParams pp{p->d_descs, t->d_pdescs,  t->d_jobs, t->head, p->d_counters + kHdrHead,
                   t->kind,       t->split,      static_cast<char*>(t->d_ws), dA, dB};
   cudaError_t e = tc_pack_launch(pp, t->pack_grid, stream);
   if (e != cudaSuccess) return cuda_error(e, "split/pack launch");
   TcGemmParams gp{p->d_descs, p->d_items,  p->n_items, p->d_counters + kHdrItems,
                   p->d_counters, t->d_tmaps, alpha,      beta,
                   dC,            t->d_err,   2000000000ull, p->d_cta_times,
-                  tc_schedule(p->mode)};
+                  tc_schedule(p->mode),
+                  t->d_pdescs,   t->pair ? t->d_jobs : nullptr,
+                  p->d_counters + kHdrHead, p->d_counters + kHdrJobs,
+                  t->d_ready,    t->cap_batch, static_cast<char*>(t->d_ws), dA, dB};
   if (p->ev_start) cudaEventRecord(p->ev_start, stream);
   e = t->pair ? tc2_gemm_launch(t->kind, t->split, gp, p->grid, stream)
               : tc_gemm_launch(t->kind, t->split, gp, p->grid, stream);
@@ -419,8 +475,9 @@ bgemm_status_t tc_check_device(bgemm_plan_s* p, cudaStream_t) {
   if (e != cudaSuccess) return cuda_error(e, "device error word");
   if (err) {
     cudaMemset(t->d_err, 0, sizeof(int));
-    // an aborted launch may have left the tile queue's counters mid-walk
-    cudaMemset(p->d_counters, 0, 2 * sizeof(int));
+    // an aborted launch may have left the queues' counters mid-walk
+    cudaMemset(p->d_counters, 0, 3 * sizeof(int));
+    cudaMemset(t->d_ready, 0, sizeof(int) * (size_t)t->cap_batch);
     return set_error(BGEMM_ERROR_DEVICE_TIMEOUT, 0, -1,
                      "a bounded wait in the tensor-core kernel expired; results are invalid");
   }
