@@ -47,8 +47,9 @@ struct FwTcScratch {
                      // bit 1: the workspace could not hold the batch (nothing ran);
                      // bit 2: no costed tile configuration (matrix skipped)
   int* gemm_err;     // bit 0: a bounded device wait of the GEMM expired
-  int* counts;       // [0] work items, [1] pre-pass strips
+  int* counts;       // [0] work items, [1] packing strips, [2] the pre-pass kernel's of them
   int* counters;     // GEMM queue counters (reset by the kernel)
+  int* ready;        // [cap_batch] strips that the GEMM kernel packed (reset by it)
   MatDesc* descs;    // [cap_batch]
   PackDesc* pdescs;  // [cap_batch]
   int* bins;         // [cap_batch] tile-time bin | K bin << 8
@@ -122,14 +123,19 @@ __host__ __device__ inline FwTcMat fwtc_plan_matrix(int M, int N, int K, int max
 
 __global__ void fwtc_plan_kernel(const int* __restrict__ dM, const int* __restrict__ dN,
                                  const int* __restrict__ dK, int batch, int max_dim, int max_k,
-                                 int mode, FwTcScratch s) {
+                                 int mode, int clusters, FwTcScratch s) {
   __shared__ int bin_tiles[kBins];
   __shared__ int bin_start[kBins];
   __shared__ int kbin_jobs[kBins];  // pre-pass strips per quarter-octave of K
   __shared__ int kbin_start[kBins];
+  __shared__ int kbin_tiles[kBins];  // and, for the division of the packing, the
+  __shared__ unsigned long long kbin_bytes[kBins], kbin_ns[kBins];  // bins' work
   __shared__ unsigned long long ws_total;
-  __shared__ int jobs_total;
-  for (int b = threadIdx.x; b < kBins; b += blockDim.x) bin_tiles[b] = kbin_jobs[b] = 0;
+  __shared__ int jobs_total, head_bin;  // bins below head_bin are the GEMM kernel's to pack
+  for (int b = threadIdx.x; b < kBins; b += blockDim.x) {
+    bin_tiles[b] = kbin_jobs[b] = kbin_tiles[b] = 0;
+    kbin_bytes[b] = kbin_ns[b] = 0;
+  }
   if (threadIdx.x == 0) {
     ws_total = 0;
     jobs_total = 0;
@@ -154,6 +160,11 @@ __global__ void fwtc_plan_kernel(const int* __restrict__ dM, const int* __restri
       pd.b_hi = (long long)(off + parts * r.a_bytes);
       pd.b_lo = parts == 2 ? (long long)(off + parts * r.a_bytes + r.b_bytes) : pd.b_hi;
       js = atomicAdd(&kbin_jobs[r.kbin], r.strips);
+      const TileCost c = c_tc_cost[mode - 1][r.desc.cfg];
+      atomicAdd(&kbin_tiles[r.kbin], r.tiles);
+      atomicAdd(&kbin_bytes[r.kbin], 4ull * (unsigned long long)(r.desc.M + r.desc.N) * r.desc.K);
+      atomicAdd(&kbin_ns[r.kbin],
+                (unsigned long long)((float)r.tiles * fmaf(c.b_ns, (float)r.desc.K, c.a_ns)));
     }
     s.pdescs[i] = pd;
     s.job_start[i] = js;
@@ -177,13 +188,33 @@ __global__ void fwtc_plan_kernel(const int* __restrict__ dM, const int* __restri
     }
     s.counts[0] = run;
     s.counts[1] = jobs_total;
+    // whole bins of K, the longest first
+    const float bytes_per_ns = (float)kFuseBytesPerNs;
+    float pack = 0.f, gemm = 0.f, late = 0.f;
+    for (int b = kBins - 1; b >= 0; --b) {
+      pack += (float)kbin_bytes[b] / bytes_per_ns;
+      late = fmaxf(late, pack - gemm);
+      gemm += (float)kbin_ns[b] / (float)clusters;
+    }
+    int b = kBins, tiles = 0, head = 0;
+    for (pack = 0.f; b > 0 && !(tiles >= kHeadTiles * clusters && pack >= late); --b) {
+      pack += (float)kbin_bytes[b - 1] / bytes_per_ns;
+      tiles += kbin_tiles[b - 1];
+      head += kbin_jobs[b - 1];
+    }
+    head_bin = b;
+    s.counts[2] = min(head, jobs_total);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < batch; i += blockDim.x) {
     const int off = s.mat_start[i];
     if (off >= 0) s.mat_start[i] = bin_start[s.bins[i] & 0xff] + off;
     const int js = s.job_start[i];
-    if (js >= 0) s.job_start[i] = kbin_start[s.bins[i] >> 8] + js;
+    if (js >= 0) {
+      const int kb = s.bins[i] >> 8;
+      s.job_start[i] = kbin_start[kb] + js;
+      if (kb < head_bin) s.pdescs[i].await = cdiv(s.descs[i].M, 32) + cdiv(s.descs[i].N, 32);
+    }
   }
 }
 
@@ -263,8 +294,11 @@ bgemm_status_t fwtc_check_device(int dev) {
     if (err[0] || err[1]) {
       cudaMemset(kv.second.s.err, 0, sizeof(int));
       cudaMemset(kv.second.s.gemm_err, 0, sizeof(int));
-      // an aborted launch may have left the tile queue's counters mid-walk
-      if (err[1]) cudaMemset(kv.second.s.counters, 0, 2 * sizeof(int));
+      // an aborted launch may have left the queues' counters mid-walk
+      if (err[1]) {
+        cudaMemset(kv.second.s.counters, 0, 3 * sizeof(int));
+        cudaMemset(kv.second.s.ready, 0, sizeof(int) * kv.second.cap_batch);
+      }
       if (err[1])
         return set_error(BGEMM_ERROR_DEVICE_TIMEOUT, 0, -1,
                          "a bounded wait in the tensor-core kernel expired; results are invalid");
@@ -359,7 +393,8 @@ extern "C" bgemm_status_t bgemm_framework_gemm_mode(const int* dM, const int* dN
     };
     const size_t o_descs = take(sizeof(MatDesc) * cb), o_pd = take(sizeof(PackDesc) * cb);
     const size_t o_bins = take(sizeof(int) * cb), o_ms = take(sizeof(int) * cb);
-    const size_t o_js = take(sizeof(int) * cb), o_items = take(sizeof(TileItem) * ci);
+    const size_t o_js = take(sizeof(int) * cb), o_ready = take(sizeof(int) * cb);
+    const size_t o_items = take(sizeof(TileItem) * ci);
     const size_t o_jobs = take(sizeof(PackJob) * cj);
     const size_t o_tm = take(sizeof(CUtensorMap) * 4 * cb);
     const size_t o_tpl = take(sizeof(CUtensorMap) * 2 * kTmapBoxClasses);
@@ -372,9 +407,12 @@ extern "C" bgemm_status_t bgemm_framework_gemm_mode(const int* dM, const int* dN
       return set_error(BGEMM_ERROR_ALLOC, 0, -1, "framework scratch of %zu bytes: %s", off,
                        cudaGetErrorString(e));
     e = cudaMemset(ctx.mem, 0, 256);
+    if (e == cudaSuccess)
+      e = cudaMemset(static_cast<char*>(ctx.mem) + o_ready, 0, sizeof(int) * cb);
     if (e != cudaSuccess) return cuda_error(e, "framework scratch init");
     char* b = static_cast<char*>(ctx.mem);
     FwTcScratch& s = ctx.s;
+    s.ready = reinterpret_cast<int*>(b + o_ready);
     s.err = reinterpret_cast<int*>(b);
     s.gemm_err = reinterpret_cast<int*>(b + 4);
     s.counts = reinterpret_cast<int*>(b + 64);
@@ -404,7 +442,8 @@ extern "C" bgemm_status_t bgemm_framework_gemm_mode(const int* dM, const int* dN
     ctx.templ = true;
   }
   const FwTcScratch s = ctx.s;
-  fwtc_plan_kernel<<<1, 1024, 0, stream>>>(dM, dN, dK, batch, max_dim, max_k, (int)mode, s);
+  fwtc_plan_kernel<<<1, 1024, 0, stream>>>(dM, dN, dK, batch, max_dim, max_k, (int)mode, clusters,
+                                           s);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_error(e, "framework plan kernel");
   fwtc_expand_kernel<<<(batch + 7) / 8, 256, 0, stream>>>(batch, s);
@@ -413,12 +452,14 @@ extern "C" bgemm_status_t bgemm_framework_gemm_mode(const int* dM, const int* dN
   TcTmapParams tp{s.descs, s.pdescs, s.templ, s.tmaps, s.ws, batch, kind, 1};
   e = tc_tmap_launch(tp, stream);
   if (e != cudaSuccess) return cuda_error(e, "tensor-map build launch");
-  TcPackParams pp{s.descs, s.pdescs, s.jobs, 0, s.counts + 1, kind, split, s.ws,
+  TcPackParams pp{s.descs, s.pdescs, s.jobs, 0, s.counts + 2, kind, split, s.ws,
                   const_cast<const float* const*>(dA), const_cast<const float* const*>(dB)};
   e = tc_pack_launch(pp, df.num_sms * kPackCtasPerSm, stream);
   if (e != cudaSuccess) return cuda_error(e, "split/pack launch");
   TcGemmParams gp{s.descs, s.items, 0, s.counts, s.counters, s.tmaps, 1.0f, 1.0f, dC,
-                  s.gemm_err, 2000000000ull, nullptr, tc_schedule(mode)};
+                  s.gemm_err, 2000000000ull, nullptr, tc_schedule(mode),
+                  s.pdescs, s.jobs, s.counts + 2, s.counts + 1, s.ready, (int)ctx.cap_batch, s.ws,
+                  const_cast<const float* const*>(dA), const_cast<const float* const*>(dB)};
   e = tc2_gemm_launch(kind, split, gp, 2 * clusters, stream);
   if (e != cudaSuccess) return cuda_error(e, "tcgen05 GEMM launch");
   return BGEMM_SUCCESS;

@@ -135,6 +135,18 @@ struct TcTmapParams {
   int pair;
 };
 
+// The division of the packing between the pre-pass kernel (the first matrices
+// of the job order) and the pair kernel's idle warps (the rest): the shortest
+// head that gives every CTA pair kHeadTiles tiles to start with and keeps each
+// later matrix's packing, at kFuseBytesPerNs of raw operands, ahead of the
+// modelled time at which its tiles begin.
+// Measured: 2, 4 and 8 tiles per pair 6.81, 6.83 and 6.88 ms (a stream of four
+// batches) and 538, 525 and 534 us (96 matrices in 3xBF16); 800, 1200 and 2000
+// bytes per ns 1283, 1230 and 1235 us (128 matrices in TF32, whose GEMM is the
+// shortest beside its packing).
+constexpr int kHeadTiles = 4;
+constexpr double kFuseBytesPerNs = 1200.0;
+
 cudaError_t tc_pack_launch(const TcPackParams& p, int grid, cudaStream_t s);
 // one CTA waiting on a barrier that never completes (bounded-wait self-test)
 cudaError_t tc_wait_selftest_launch(int* err, int* out, unsigned long long limit_ns,

@@ -174,17 +174,7 @@ static long long tc_tiles(const MatDesc& d, bool pair) {
   const int bm = pair ? 256 : kTcBM, bn = pair ? tc2_cfg_bn(d.cfg) : tc_cfg_bn(d.cfg);
   return cdiv(swap ? d.N : d.M, bm) * cdiv(swap ? d.M : d.N, bn);
 }
-// The division of the packing between the pre-pass kernel (the first matrices
-// of the job order) and the pair kernel's idle warps (the rest): the shortest
-// head that gives every CTA pair kHeadTiles tiles to start with and keeps each
-// later matrix's packing, at kFuseBytesPerNs of raw operands, ahead of the
-// modelled time at which its tiles begin.  Returns the number of jobs.
-// Measured: 2, 4 and 8 tiles per pair 6.81, 6.83 and 6.88 ms (a stream of four
-// batches) and 538, 525 and 534 us (96 matrices in 3xBF16); 800, 1200 and 2000
-// bytes per ns 1283, 1230 and 1235 us (128 matrices in TF32, whose GEMM is the
-// shortest beside its packing).
-constexpr int kHeadTiles = 4;
-constexpr double kFuseBytesPerNs = 1200.0;
+// Jobs of the pre-pass kernel (the rule is in tc_common.h).
 static int tc_divide(TcPlan* t, const std::vector<MatDesc>& hd, const std::vector<int>& order) {
   if (!t->pair) return (int)t->jobs.size();
   // packing done and GEMM begun, in ns from the GEMM kernel's start, if all

@@ -85,3 +85,26 @@ def test_packing_in_the_gemm_3xtf32(cuda, layout, ta, tb, pad):
 @pytest.mark.parametrize("mode", ["tf32", "bf16x3", "tf32x3"])
 def test_packing_in_the_gemm_modes(cuda, mode):
     check(mode, "col", False, False, 1, *sizes(5), alpha=-0.5, beta=1.0)
+
+
+@pytest.mark.parametrize("mode", ["tf32", "bf16x3", "tf32x3"])
+def test_packing_in_the_gemm_device_sizes(cuda, mode):
+    """The device-size entry divides the packing on the device (C += A B)."""
+    M, N, K = sizes(9)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    mats = [[torch.empty((c, r), device="cuda").uniform_(-1, 1, generator=gen).t()
+             for r, c in zip(x, y)] for x, y in ((M, K), (K, N), (M, N))]
+    c0 = [c.t().clone().t() for c in mats[2]]
+    dev = [torch.tensor(v, dtype=torch.int32, device="cuda") for v in (M, N, K)]
+    ptr = [torch.tensor([m.data_ptr() for m in x], device="cuda") for x in mats]
+    factor, unit = BOUND[mode]
+    for _ in range(2):
+        for c, o in zip(mats[2], c0):
+            c.copy_(o)
+        bg.framework_gemm_mode(*(v.data_ptr() for v in dev), *(v.data_ptr() for v in ptr), len(M),
+                               300, 257, mode=mode)
+        bg.framework_check_device()
+        for a, b, c, o, k in zip(*mats, c0, K):
+            a, b, o = a.double(), b.double(), o.double()
+            bound = factor * unit * max(k, 1) ** 0.5 * (a.abs() @ b.abs() + o.abs()) + 1e-30
+            assert bool(((c.double() - (a @ b + o)).abs() <= bound).all())
