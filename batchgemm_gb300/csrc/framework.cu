@@ -51,61 +51,70 @@ __host__ __device__ inline int fw_bin(int K, TileCost t) {
   return q < 0 ? 0 : q > kBins - 1 ? kBins - 1 : q;
 }
 
-// One thread per matrix (in turns).  The sums of every limit step are formed
-// in one pass: a matrix's candidates are modelled once and picked from
-// kSimtSteps + 1 times.
+// One thread per matrix (in turns).  One CTA, so its latency counts, not its
+// throughput: the sums of every limit step are formed in one pass (a matrix's
+// candidates are modelled once and picked from kSimtSteps times), per warp
+// without atomics; the bins' prefix sums run in parallel (16.5 us with 64-bit
+// shared atomics and one thread's loop over the bins, for 256 matrices).
 __global__ void __launch_bounds__(kPlanThreads)
     fw_plan_kernel(const int* __restrict__ dM, const int* __restrict__ dN,
                    const int* __restrict__ dK, int batch, int max_dim, int slots, FwScratch s) {
+  constexpr int kPlanWarps = kPlanThreads / 32;
   __shared__ int bin_tiles[kBins];
   __shared__ int bin_start[kBins];
-  __shared__ unsigned long long work[kSimtSteps + 1];
-  __shared__ int longest[kSimtSteps + 1];  // non-negative floats order as ints
+  __shared__ long long work_w[kPlanWarps][kSimtSteps + 1];
+  __shared__ float longest_w[kPlanWarps][kSimtSteps + 1];
+  __shared__ long long work[kSimtSteps + 1];
+  __shared__ float longest[kSimtSteps + 1];
   __shared__ float limit;
-  for (int b = threadIdx.x; b < kBins; b += blockDim.x) bin_tiles[b] = 0;
-  if (threadIdx.x <= kSimtSteps) {
-    work[threadIdx.x] = 0;
-    longest[threadIdx.x] = 0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x < kBins) bin_tiles[threadIdx.x] = 0;
+  if (lane <= kSimtSteps) {
+    work_w[warp][lane] = 0;
+    longest_w[warp][lane] = 0.0f;
   }
-  __syncthreads();
+  __syncwarp();
+  // steps from .. to, each warp's part
   auto sums = [&](int from, int to) {
-    for (int i0 = 0; i0 < batch; i0 += blockDim.x) {
-      const int i = i0 + threadIdx.x;
+    for (int i0 = warp * 32; i0 < batch; i0 += kPlanThreads) {
+      const int i = i0 + lane;
       const int M = i < batch ? dM[i] : 0, N = i < batch ? dN[i] : 0, K = i < batch ? dK[i] : 0;
       const bool any = !fw_bad(M, N, K, max_dim) && M > 0 && N > 0;
       SimtCands e;
       if (any) simt_cands(M, N, K, -1, c_cfgs, c_cost, &e);
+      float T = from == 0 ? 3e38f : longest[0];
       for (int j = from; j <= to; ++j) {
+        if (j > 0) T *= 0.70710678f;
         float w = 0.0f, l = 0.0f;
-        if (any) {
-          const float T = j == 0 ? 3e38f : simt_limit(__int_as_float(longest[0]), j);
-          if (simt_pick(e, T, &w, &l) < 0) w = l = 0.0f;
-        }
+        if (any && simt_pick(e, T, &w, &l) < 0) w = l = 0.0f;
         long long v = (long long)w;
-        int m = __float_as_int(l);
         for (int o = 16; o; o >>= 1) {
           v += __shfl_xor_sync(0xffffffffu, v, o);
-          m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+          l = fmaxf(l, __shfl_xor_sync(0xffffffffu, l, o));
         }
-        if ((threadIdx.x & 31) == 0 && m > 0) {
-          atomicAdd(&work[j], (unsigned long long)v);
-          atomicMax(&longest[j], m);
+        if (lane == 0) {
+          work_w[warp][j] += v;
+          longest_w[warp][j] = fmaxf(longest_w[warp][j], l);
         }
       }
+    }
+    __syncthreads();
+    if (threadIdx.x >= from && threadIdx.x <= to) {
+      long long v = 0;
+      float l = 0.0f;
+#pragma unroll 8
+      for (int w = 0; w < kPlanWarps; ++w) {
+        v += work_w[w][threadIdx.x];
+        l = fmaxf(l, longest_w[w][threadIdx.x]);
+      }
+      work[threadIdx.x] = v;
+      longest[threadIdx.x] = l;
     }
     __syncthreads();
   };
   sums(0, 0);
   sums(1, kSimtSteps);
-  if (threadIdx.x == 0) {
-    long long w[kSimtSteps + 1];
-    float l[kSimtSteps + 1];
-    for (int j = 0; j <= kSimtSteps; ++j) {
-      w[j] = (long long)work[j];
-      l[j] = __int_as_float(longest[j]);
-    }
-    limit = simt_choose_limit(w, l, slots);
-  }
+  if (threadIdx.x == 0) limit = simt_choose_limit(work, longest, slots);
   __syncthreads();
   // each matrix reserves its tiles in the bin of its tile time
   for (int i = threadIdx.x; i < batch; i += blockDim.x) {
@@ -129,13 +138,12 @@ __global__ void __launch_bounds__(kPlanThreads)
     s.mat_start[i] = start;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < kBins) {  // longest tiles first
     int run = 0;
-    for (int b = kBins - 1; b >= 0; --b) {  // longest tiles first
-      bin_start[b] = run;
-      run += bin_tiles[b];
-    }
-    *s.n_items = run;
+#pragma unroll 16
+    for (int b = 0; b < kBins; ++b) run += b > (int)threadIdx.x ? bin_tiles[b] : 0;
+    bin_start[threadIdx.x] = run;
+    if (threadIdx.x == 0) *s.n_items = run + bin_tiles[0];
   }
   __syncthreads();
   for (int i = threadIdx.x; i < batch; i += blockDim.x) {

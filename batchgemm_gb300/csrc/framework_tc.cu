@@ -128,33 +128,50 @@ __global__ void fwtc_plan_kernel(const int* __restrict__ dM, const int* __restri
   __shared__ int bin_start[kBins];
   __shared__ int kbin_jobs[kBins];  // pre-pass strips per quarter-octave of K
   __shared__ int kbin_start[kBins];
-  __shared__ int kbin_tiles[kBins];  // and, for the division of the packing, the
-  __shared__ unsigned long long kbin_bytes[kBins], kbin_ns[kBins];  // bins' work
+  // for the division of the packing: the bins' tiles, raw KB and tile time (64
+  // ns units; 32-bit, as 64-bit shared atomics are compare-and-swap loops: with
+  // them the kernel took 66 us for 1000 matrices)
+  __shared__ int kbin_tiles[kBins], kbin_kb[kBins], kbin_time[kBins];
   __shared__ unsigned long long ws_total;
-  __shared__ int jobs_total, head_bin;  // bins below head_bin are the GEMM kernel's to pack
-  for (int b = threadIdx.x; b < kBins; b += blockDim.x) {
-    bin_tiles[b] = kbin_jobs[b] = kbin_tiles[b] = 0;
-    kbin_bytes[b] = kbin_ns[b] = 0;
-  }
+  __shared__ int head_bin;  // bins below it are the GEMM kernel's to pack
+  __shared__ float late_w[kBins / 32];
+  if (threadIdx.x < kBins)
+    bin_tiles[threadIdx.x] = kbin_jobs[threadIdx.x] = kbin_tiles[threadIdx.x] =
+        kbin_kb[threadIdx.x] = kbin_time[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
     ws_total = 0;
-    jobs_total = 0;
+    head_bin = 0;
   }
   __syncthreads();
   const int parts = (mode == BGEMM_MODE_TF32) ? 1 : 2;
-  for (int i = threadIdx.x; i < batch; i += blockDim.x) {
-    const FwTcMat r = fwtc_plan_matrix(dM[i], dN[i], dK[i], max_dim, max_k, mode,
-                                       c_tc_cost[mode - 1]);
-    if (r.bad) atomicOr(s.err, 1);
-    if (r.nocfg) atomicOr(s.err, 4);
-    s.descs[i] = r.desc;
-    s.mat_start[i] = r.tiles ? atomicAdd(&bin_tiles[r.bin], r.tiles) : -1;
-    // split-operand panels and pre-pass strips of a matrix with work
+  const int lane = threadIdx.x & 31;
+  for (int i0 = threadIdx.x - lane; i0 < batch; i0 += blockDim.x) {
+    const int i = i0 + lane;
+    const bool in = i < batch;
+    FwTcMat r{};
+    if (in) {
+      r = fwtc_plan_matrix(dM[i], dN[i], dK[i], max_dim, max_k, mode, c_tc_cost[mode - 1]);
+      if (r.bad) atomicOr(s.err, 1);
+      if (r.nocfg) atomicOr(s.err, 4);
+      s.descs[i] = r.desc;
+      s.mat_start[i] = r.tiles ? atomicAdd(&bin_tiles[r.bin], r.tiles) : -1;
+    }
+    // split-operand panels (one reservation per warp) and packing strips of the
+    // matrices with work
+    const unsigned long long bytes = r.strips ? parts * (r.a_bytes + r.b_bytes) : 0;
+    unsigned long long end = bytes;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long v = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += v;
+    }
+    unsigned long long off = 0;
+    if (lane == 31 && end) off = atomicAdd(&ws_total, end);
+    off = __shfl_sync(0xffffffffu, off, 31) + end - bytes;
+    if (!in) continue;
     PackDesc pd{};
     pd.kpad = r.kpad;
     int js = -1;
     if (r.strips) {
-      const unsigned long long off = atomicAdd(&ws_total, parts * (r.a_bytes + r.b_bytes));
       pd.a_hi = (long long)off;
       pd.a_lo = parts == 2 ? (long long)(off + r.a_bytes) : pd.a_hi;
       pd.b_hi = (long long)(off + parts * r.a_bytes);
@@ -162,50 +179,53 @@ __global__ void fwtc_plan_kernel(const int* __restrict__ dM, const int* __restri
       js = atomicAdd(&kbin_jobs[r.kbin], r.strips);
       const TileCost c = c_tc_cost[mode - 1][r.desc.cfg];
       atomicAdd(&kbin_tiles[r.kbin], r.tiles);
-      atomicAdd(&kbin_bytes[r.kbin], 4ull * (unsigned long long)(r.desc.M + r.desc.N) * r.desc.K);
-      atomicAdd(&kbin_ns[r.kbin],
-                (unsigned long long)((float)r.tiles * fmaf(c.b_ns, (float)r.desc.K, c.a_ns)));
+      atomicAdd(&kbin_kb[r.kbin],
+                (int)((4ll * ((long long)r.desc.M + r.desc.N) * r.desc.K + 1023) >> 10));
+      atomicAdd(&kbin_time[r.kbin],
+                (int)((float)r.tiles * fmaf(c.b_ns, (float)r.desc.K, c.a_ns) * (1.0f / 64.0f)));
     }
     s.pdescs[i] = pd;
     s.job_start[i] = js;
     s.bins[i] = r.bin | (r.kbin << 8);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  // per bin: queue slots of longer tiles, strips of longer K, and the packing
+  // and GEMM time up to it
+  float pack = 0.f, gemm = 0.f, late = 0.f;
+  int tiles = 0, jobs = 0;
+  if (threadIdx.x < kBins) {
+    const int me = threadIdx.x;
     int run = 0;
-    for (int b = kBins - 1; b >= 0; --b) {  // longest tiles first
-      bin_start[b] = run;
-      run += bin_tiles[b];
-    }
-    for (int b = kBins - 1; b >= 0; --b) {  // strips of the longest K first
-      kbin_start[b] = jobs_total;
-      jobs_total += kbin_jobs[b];
-    }
-    if (ws_total > s.cap_ws) {
-      atomicOr(s.err, 2);
-      run = 0;
-      jobs_total = 0;
-    }
-    s.counts[0] = run;
-    s.counts[1] = jobs_total;
-    // whole bins of K, the longest first
-    const float bytes_per_ns = (float)kFuseBytesPerNs;
-    float pack = 0.f, gemm = 0.f, late = 0.f;
+#pragma unroll 8
     for (int b = kBins - 1; b >= 0; --b) {
-      pack += (float)kbin_bytes[b] / bytes_per_ns;
-      late = fmaxf(late, pack - gemm);
-      gemm += (float)kbin_ns[b] / (float)clusters;
+      run += b > me ? bin_tiles[b] : 0;
+      if (b >= me) {
+        pack += (float)kbin_kb[b] * (float)(1024.0 / kFuseBytesPerNs);
+        tiles += kbin_tiles[b];
+        jobs += kbin_jobs[b];
+      }
+      if (b > me) gemm += (float)kbin_time[b] * (64.0f / (float)clusters);
     }
-    int b = kBins, tiles = 0, head = 0;
-    for (pack = 0.f; b > 0 && !(tiles >= kHeadTiles * clusters && pack >= late); --b) {
-      pack += (float)kbin_bytes[b - 1] / bytes_per_ns;
-      tiles += kbin_tiles[b - 1];
-      head += kbin_jobs[b - 1];
+    bin_start[me] = run;
+    kbin_start[me] = jobs - kbin_jobs[me];
+    late = pack - gemm;
+    for (int o = 16; o; o >>= 1) late = fmaxf(late, __shfl_xor_sync(0xffffffffu, late, o));
+    if (lane == 0) late_w[me >> 5] = late;
+    if (me == 0) {
+      const bool fits = ws_total <= s.cap_ws;
+      if (!fits) atomicOr(s.err, 2);
+      s.counts[0] = fits ? run + bin_tiles[0] : 0;
+      s.counts[1] = fits ? jobs : 0;
+      s.counts[2] = fits ? jobs : 0;
     }
-    head_bin = b;
-    s.counts[2] = min(head, jobs_total);
   }
   __syncthreads();
+  if (threadIdx.x < kBins) {
+    late = fmaxf(0.f, fmaxf(late_w[0], late_w[1]));
+    if (tiles >= kHeadTiles * clusters && pack >= late) atomicMax(&head_bin, (int)threadIdx.x);
+  }
+  __syncthreads();
+  if (threadIdx.x == head_bin && s.counts[1] > 0) s.counts[2] = jobs;
   for (int i = threadIdx.x; i < batch; i += blockDim.x) {
     const int off = s.mat_start[i];
     if (off >= 0) s.mat_start[i] = bin_start[s.bins[i] & 0xff] + off;

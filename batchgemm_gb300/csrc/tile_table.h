@@ -176,17 +176,17 @@ __host__ __device__ inline float simt_limit(float longest, int step) {
 }
 __host__ __device__ inline float simt_choose_limit(const long long* work, const float* longest,
                                                    int slots) {
-  float best = 0.0f;
-  int at = 0;
+  float best = 0.0f, limit = longest[0], T = 3e38f;  // limit: step j - 1's
   for (int j = 0; j <= kSimtSteps; ++j) {
-    if (j > 0 && kSimtTail * simt_limit(longest[0], j - 1) <= 0.02f * best) break;
+    if (j > 0 && kSimtTail * limit <= 0.02f * best) break;
+    if (j > 0) limit *= 0.70710678f;
     const float m = fmaf(kSimtTail, longest[j], (float)work[j] / (float)slots);
     if (j == 0 || m < best) {
       best = m;
-      at = j;
+      T = j == 0 ? 3e38f : limit;
     }
   }
-  return at == 0 ? 3e38f : simt_limit(longest[0], at);
+  return T;
 }
 
 }  // namespace bgemm
