@@ -42,6 +42,35 @@ struct TileItem {
                     // orientation: along the MMA's M and N)
 };
 
+// ------------------------------------------- programmatic dependent launch --
+// The kernels of one call follow one another in a stream.  A kernel launched
+// with pdl_launch may be set up once every CTA of the kernel before it has
+// passed pdl_trigger() (or ended); all it does with memory stands behind its
+// pdl_wait(), which waits for the end of that kernel.  So only the launch and
+// the set-up overlap, about 2 us per kernel.
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+cudaError_t pdl_launch(void (*kernel)(Params...), int grid, int threads, size_t smem,
+                       cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid, 1, 1);
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+#endif
+
 // ---------------------------------------------------------------- SIMT ----
 // Tile configurations of the FP32 SIMT kernel.  The 128 x 128 tile (id 7) and
 // the thin ones (ids 8 and 9, for M <= 8 and N <= 8) are computed by a CTA of
@@ -88,6 +117,8 @@ struct SimtParams {
 // ta / tb: the plan's matrices carry kTransAFlag / kTransBFlag
 cudaError_t simt_launch(const SimtParams& p, int grid, cudaStream_t stream, bool ta = false,
                         bool tb = false);
+// behind a kernel that triggers (the device planner's)
+cudaError_t simt_launch_behind(const SimtParams& p, int grid, cudaStream_t stream);
 int simt_ctas_per_sm();
 
 }  // namespace bgemm

@@ -67,6 +67,7 @@ __global__ void __launch_bounds__(kPlanThreads)
   __shared__ long long work[kSimtSteps + 1];
   __shared__ float longest[kSimtSteps + 1];
   __shared__ float limit;
+  pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x < kBins) bin_tiles[threadIdx.x] = 0;
   if (lane <= kSimtSteps) {
@@ -153,6 +154,8 @@ __global__ void __launch_bounds__(kPlanThreads)
 }
 
 __global__ void fw_expand_kernel(int batch, FwScratch s) {
+  pdl_trigger();
+  pdl_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= batch) return;
@@ -248,12 +251,11 @@ extern "C" bgemm_status_t bgemm_framework_gemm(const int* dM, const int* dN, con
   fw_plan_kernel<<<1, kPlanThreads, 0, stream>>>(dM, dN, dK, batch, max_dim, grid, ctx.s);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_error(e, "framework plan kernel");
-  fw_expand_kernel<<<(batch + 7) / 8, 256, 0, stream>>>(batch, ctx.s);
-  e = cudaGetLastError();
+  e = pdl_launch(fw_expand_kernel, (batch + 7) / 8, 256, 0, stream, batch, ctx.s);
   if (e != cudaSuccess) return cuda_error(e, "framework expand kernel");
   SimtParams sp{ctx.s.descs, ctx.s.items, 0, ctx.s.n_items, ctx.s.counters, 1.0f, 1.0f,
                 const_cast<const float* const*>(dA), const_cast<const float* const*>(dB), dC};
-  e = simt_launch(sp, grid, stream);
+  e = simt_launch_behind(sp, grid, stream);
   if (e != cudaSuccess) return cuda_error(e, "framework SIMT launch");
   return BGEMM_SUCCESS;
 }
@@ -303,12 +305,11 @@ cudaError_t fw_launch_on_scratch(const int* dM, const int* dN, const int* dK, fl
   fw_plan_kernel<<<1, kPlanThreads, 0, stream>>>(dM, dN, dK, batch, max_dim, grid, s);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  fw_expand_kernel<<<(batch + 7) / 8, 256, 0, stream>>>(batch, s);
-  e = cudaGetLastError();
+  e = pdl_launch(fw_expand_kernel, (batch + 7) / 8, 256, 0, stream, batch, s);
   if (e != cudaSuccess) return e;
   SimtParams sp{s.descs, s.items, 0, s.n_items, s.counters, 1.0f, 1.0f,
                 const_cast<const float* const*>(dA), const_cast<const float* const*>(dB), dC};
-  return simt_launch(sp, grid, stream);
+  return simt_launch_behind(sp, grid, stream);
 }
 
 }  // namespace bgemm

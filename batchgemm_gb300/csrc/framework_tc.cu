@@ -135,6 +135,7 @@ __global__ void fwtc_plan_kernel(const int* __restrict__ dM, const int* __restri
   __shared__ unsigned long long ws_total;
   __shared__ int head_bin;  // bins below it are the GEMM kernel's to pack
   __shared__ float late_w[kBins / 32];
+  pdl_trigger();
   if (threadIdx.x < kBins)
     bin_tiles[threadIdx.x] = kbin_jobs[threadIdx.x] = kbin_tiles[threadIdx.x] =
         kbin_kb[threadIdx.x] = kbin_time[threadIdx.x] = 0;
@@ -239,6 +240,8 @@ __global__ void fwtc_plan_kernel(const int* __restrict__ dM, const int* __restri
 }
 
 __global__ void fwtc_expand_kernel(int batch, FwTcScratch s) {
+  pdl_trigger();
+  pdl_wait();
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (i >= batch || s.counts[0] == 0) return;
@@ -466,15 +469,14 @@ extern "C" bgemm_status_t bgemm_framework_gemm_mode(const int* dM, const int* dN
                                            s);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_error(e, "framework plan kernel");
-  fwtc_expand_kernel<<<(batch + 7) / 8, 256, 0, stream>>>(batch, s);
-  e = cudaGetLastError();
+  e = pdl_launch(fwtc_expand_kernel, (batch + 7) / 8, 256, 0, stream, batch, s);
   if (e != cudaSuccess) return cuda_error(e, "framework expand kernel");
   TcTmapParams tp{s.descs, s.pdescs, s.templ, s.tmaps, s.ws, batch, kind, 1};
-  e = tc_tmap_launch(tp, stream);
+  e = tc_tmap_launch(tp, stream, true);
   if (e != cudaSuccess) return cuda_error(e, "tensor-map build launch");
   TcPackParams pp{s.descs, s.pdescs, s.jobs, 0, s.counts + 2, kind, split, s.ws,
                   const_cast<const float* const*>(dA), const_cast<const float* const*>(dB)};
-  e = tc_pack_launch(pp, df.num_sms * kPackCtasPerSm, stream);
+  e = tc_pack_launch(pp, df.num_sms * kPackCtasPerSm, stream, true);
   if (e != cudaSuccess) return cuda_error(e, "split/pack launch");
   TcGemmParams gp{s.descs, s.items, 0, s.counts, s.counters, s.tmaps, 1.0f, 1.0f, dC,
                   s.gemm_err, 2000000000ull, nullptr, tc_schedule(mode),

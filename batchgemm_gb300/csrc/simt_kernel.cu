@@ -25,20 +25,30 @@ cudaError_t simt_launch_tn(const SimtParams& p, int grid, cudaStream_t stream);
 cudaError_t simt_launch_nt(const SimtParams& p, int grid, cudaStream_t stream);
 cudaError_t simt_launch_tt(const SimtParams& p, int grid, cudaStream_t stream);
 
+static cudaError_t simt_attributes() {
+  static bool done = false;
+  if (done) return cudaSuccess;
+  const cudaError_t e =
+      cudaFuncSetAttribute(simt_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           simt::kSmemBytes);
+  done = e == cudaSuccess;
+  return e;
+}
+
 cudaError_t simt_launch(const SimtParams& p, int grid, cudaStream_t stream, bool ta, bool tb) {
   if (ta && tb) return simt_launch_tt(p, grid, stream);
   if (ta) return simt_launch_tn(p, grid, stream);
   if (tb) return simt_launch_nt(p, grid, stream);
-  static bool attr_done = false;
-  if (!attr_done) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(simt_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             simt::kSmemBytes);
-    if (e != cudaSuccess) return e;
-    attr_done = true;
-  }
+  const cudaError_t e = simt_attributes();
+  if (e != cudaSuccess) return e;
   simt_persistent_kernel<<<grid, simt::kThreads, simt::kSmemBytes, stream>>>(p);
   return cudaGetLastError();
+}
+
+cudaError_t simt_launch_behind(const SimtParams& p, int grid, cudaStream_t stream) {
+  const cudaError_t e = simt_attributes();
+  if (e != cudaSuccess) return e;
+  return pdl_launch(simt_persistent_kernel, grid, simt::kThreads, simt::kSmemBytes, stream, p);
 }
 
 int simt_ctas_per_sm() {

@@ -604,6 +604,7 @@ __device__ __noinline__ int run_tile(const SimtParams& p, int mat, int m0, int n
 // after the tile they are at, and the CTA computes what was left together.
 template <bool TA, bool TB>
 __device__ __forceinline__ void persistent_body(const SimtParams& p) {
+  pdl_wait();
   volatile int* ctl = control();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_items = p.n_items_dev ? *p.n_items_dev : p.n_items;

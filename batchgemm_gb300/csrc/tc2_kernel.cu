@@ -326,11 +326,9 @@ __global__ void __launch_bounds__(kThreads2, 1) tc2_gemm_kernel(const TcGemmPara
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int n_items = p.n_items_dev ? *p.n_items_dev : p.n_items;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int ncl = gridDim.x >> 1;
-  if (p.cta_times && threadIdx.x == 0) p.cta_times[2 * blockIdx.x] = gtimer();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kS; ++s) {
@@ -359,6 +357,9 @@ __global__ void __launch_bounds__(kThreads2, 1) tc2_gemm_kernel(const TcGemmPara
   cluster_sync();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  pdl_wait();  // (all of the above runs beside the pre-pass's last CTAs)
+  const int n_items = p.n_items_dev ? *p.n_items_dev : p.n_items;
+  if (p.cta_times && threadIdx.x == 0) p.cta_times[2 * blockIdx.x] = gtimer();
 
   // Each warpgroup sets its register budget at one point that all four of
   // its warps execute (setmaxnreg is warpgroup-aligned), ahead of the roles'
@@ -754,13 +755,15 @@ cudaError_t launch2(const TcGemmParams& p, int grid, cudaStream_t s) {
   cfg.blockDim = dim3(kThreads2, 1, 1);
   cfg.dynamicSmemBytes = Geo2<SPLIT>::SMEM;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 2;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, tc2_gemm_kernel<KIND, SPLIT, BETA>, p);
 }
 

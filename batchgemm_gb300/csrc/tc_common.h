@@ -147,14 +147,16 @@ struct TcTmapParams {
 constexpr int kHeadTiles = 4;
 constexpr double kFuseBytesPerNs = 1200.0;
 
-cudaError_t tc_pack_launch(const TcPackParams& p, int grid, cudaStream_t s);
+// behind: the kernel before it on the stream triggers (pdl_trigger)
+cudaError_t tc_pack_launch(const TcPackParams& p, int grid, cudaStream_t s, bool behind = false);
 // one CTA waiting on a barrier that never completes (bounded-wait self-test)
 cudaError_t tc_wait_selftest_launch(int* err, int* out, unsigned long long limit_ns,
                                     cudaStream_t s);
-cudaError_t tc_tmap_launch(const TcTmapParams& p, cudaStream_t s);
+cudaError_t tc_tmap_launch(const TcTmapParams& p, cudaStream_t s, bool behind = false);
 cudaError_t tc_gemm_launch(int kind, int split, const TcGemmParams& p, int grid, cudaStream_t s);
 int tc_smem_bytes(int kind, int split);
-// CTA-pair kernel; grid = 2 x clusters
+// CTA-pair kernel; grid = 2 x clusters.  Both GEMM kernels go behind the
+// pre-pass, which triggers.
 cudaError_t tc2_gemm_launch(int kind, int split, const TcGemmParams& p, int grid,
                             cudaStream_t s);
 int tc2_max_clusters();

@@ -83,6 +83,8 @@ constexpr int kPackK = 256;
 template <int KIND, int SPLIT>
 __global__ void __launch_bounds__(256) tc_pack_kernel(const TcPackParams p) {
   __shared__ float t[kPackK][33];
+  pdl_trigger();
+  pdl_wait();
   const int tid = threadIdx.x;
   const int n_jobs = p.n_jobs_dev ? *p.n_jobs_dev : p.n_jobs;
   for (int j = blockIdx.x; j < n_jobs; j += gridDim.x) {
@@ -209,6 +211,8 @@ __global__ void __launch_bounds__(128) tc_tmap_kernel(const TcTmapParams p) {
   __shared__ __align__(128) CUtensorMap maps[4];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int j = blockIdx.x * 4 + warp;
+  pdl_trigger();
+  pdl_wait();
   if (j >= 4 * p.batch) return;
   const int i = j >> 2, part = j & 3;
   const MatDesc d = p.descs[i];
@@ -266,9 +270,6 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const TcGemmParams
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int n_items = p.n_items_dev ? *p.n_items_dev : p.n_items;
-  if (p.cta_times && threadIdx.x == 0) p.cta_times[2 * blockIdx.x] = gtimer();
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
       mbar_init(full(s), 1);
@@ -294,6 +295,9 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const TcGemmParams
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  pdl_wait();  // (all of the above runs beside the pre-pass's last CTAs)
+  const int n_items = p.n_items_dev ? *p.n_items_dev : p.n_items;
+  if (p.cta_times && threadIdx.x == 0) p.cta_times[2 * blockIdx.x] = gtimer();
 
   if (warp == 0) {
     // ------------------------------------------------ producer + scheduler
@@ -565,8 +569,7 @@ cudaError_t launch_gemm(const TcGemmParams& p, int grid, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     attr = true;
   }
-  tc_gemm_kernel<KIND, SPLIT><<<grid, kThreads, bytes, s>>>(p);
-  return cudaGetLastError();
+  return pdl_launch(tc_gemm_kernel<KIND, SPLIT>, grid, kThreads, bytes, s, p);
 }
 
 // Self-test of the bounded mbarrier wait every tensor-core kernel uses: one
@@ -598,21 +601,24 @@ cudaError_t tc_wait_selftest_launch(int* err, int* out, unsigned long long limit
   return cudaGetLastError();
 }
 
-cudaError_t tc_tmap_launch(const TcTmapParams& p, cudaStream_t s) {
+cudaError_t tc_tmap_launch(const TcTmapParams& p, cudaStream_t s, bool behind) {
   if (p.batch == 0) return cudaSuccess;
+  if (behind) return pdl_launch(tc_tmap_kernel, p.batch, 128, 0, s, p);
   tc_tmap_kernel<<<p.batch, 128, 0, s>>>(p);  // 4 warps = the 4 maps of one matrix
   return cudaGetLastError();
 }
 
-cudaError_t tc_pack_launch(const TcPackParams& p, int grid, cudaStream_t s) {
-  if (p.n_jobs == 0 && !p.n_jobs_dev) return cudaSuccess;
-  if (p.kind == kKindBF16)
-    tc_pack_kernel<kKindBF16, 1><<<grid, 256, 0, s>>>(p);
-  else if (p.split)
-    tc_pack_kernel<kKindTF32, 1><<<grid, 256, 0, s>>>(p);
-  else
-    tc_pack_kernel<kKindTF32, 0><<<grid, 256, 0, s>>>(p);
+template <int KIND, int SPLIT>
+cudaError_t launch_pack(const TcPackParams& p, int grid, cudaStream_t s, bool behind) {
+  if (behind) return pdl_launch(tc_pack_kernel<KIND, SPLIT>, grid, 256, 0, s, p);
+  tc_pack_kernel<KIND, SPLIT><<<grid, 256, 0, s>>>(p);
   return cudaGetLastError();
+}
+cudaError_t tc_pack_launch(const TcPackParams& p, int grid, cudaStream_t s, bool behind) {
+  if (p.n_jobs == 0 && !p.n_jobs_dev) return cudaSuccess;
+  if (p.kind == kKindBF16) return launch_pack<kKindBF16, 1>(p, grid, s, behind);
+  return p.split ? launch_pack<kKindTF32, 1>(p, grid, s, behind)
+                 : launch_pack<kKindTF32, 0>(p, grid, s, behind);
 }
 
 cudaError_t tc_gemm_launch(int kind, int split, const TcGemmParams& p, int grid, cudaStream_t s) {
