@@ -117,10 +117,11 @@ __host__ __device__ inline float simt_tile_ns(int K, TileCost t) {
 }
 // The time a tile takes itself, with the SM nearly to itself, as the last ones
 // run (measured on thin matrices of K = 4096: 38, 55, 94, 33 and 30 ns per k
-// for ids 0, 1, 7, 8, 9; the 128 x 128 tile between that and its busy 219 ns).
+// for ids 0, 1, 7, 8, 9, the 128 x 128 tile between that and its busy 219 ns;
+// on 16 matrices of at most 32: 2.4 us a tile of id 0 and 3.6 of id 1).
 __host__ __device__ inline float simt_alone_ns(int K, TileCost t, int c) {
   const float f = c == 0 ? 4.5f : c < 7 ? 3.0f : c == 7 ? 0.6f : 0.75f;
-  return fmaf(t.b_ns * f, (float)K, t.a_ns * (c < 7 ? 3.0f : f));
+  return fmaf(t.b_ns * f, (float)K, t.a_ns * (c == 0 ? 3.0f : c < 7 ? 4.5f : f));
 }
 // All tiles of a matrix.  A ragged edge's FMAs are skipped in steps of gm x gn
 // outputs, its copies are not.
