@@ -51,92 +51,123 @@ __host__ __device__ inline int fw_bin(int K, TileCost t) {
   return q < 0 ? 0 : q > kBins - 1 ? kBins - 1 : q;
 }
 
-// One thread per matrix (in turns).  One CTA, so its latency counts, not its
-// throughput: the sums of every limit step are formed in one pass (a matrix's
-// candidates are modelled once and picked from kSimtSteps times), per warp
-// without atomics; the bins' prefix sums run in parallel (16.5 us with 64-bit
-// shared atomics and one thread's loop over the bins, for 256 matrices).
+// Sum of a 64-bit value over the warp, in pieces that 32 lanes cannot overflow.
+__device__ __forceinline__ long long warp_sum(long long v) {
+  const unsigned long long u = (unsigned long long)v;
+  const unsigned m = (1u << 27) - 1;
+  const unsigned long long a = __reduce_add_sync(0xffffffffu, (unsigned)u & m);
+  const unsigned long long b = __reduce_add_sync(0xffffffffu, (unsigned)(u >> 27) & m);
+  const unsigned long long c = __reduce_add_sync(0xffffffffu, (unsigned)(u >> 54));
+  return (long long)(a + (b << 27) + (c << 54));
+}
+
+// One thread per matrix.  One CTA, so its latency counts, not its throughput:
+// a matrix's candidates are modelled once and stay in registers (in batches of
+// more than kPlanThreads, where a thread takes several in turn, once a pass);
+// the sums of every limit step are formed in one pass, per warp without
+// atomics; warps that a small batch leaves idle share the steps; the bins'
+// prefix sums run in parallel.  256 matrices: 16.5 us with 64-bit shared
+// atomics and one thread's loop over the bins, 12.6 with all steps in the
+// eight warps that had matrices and the candidates modelled three times,
+// 9.1 as it is.
 __global__ void __launch_bounds__(kPlanThreads)
     fw_plan_kernel(const int* __restrict__ dM, const int* __restrict__ dN,
                    const int* __restrict__ dK, int batch, int max_dim, int slots, FwScratch s) {
   constexpr int kPlanWarps = kPlanThreads / 32;
+  static_assert(kPlanWarps == 32 && kSimtSteps < 32, "a warp per step, a lane per warp");
   __shared__ int bin_tiles[kBins];
   __shared__ int bin_start[kBins];
   __shared__ long long work_w[kPlanWarps][kSimtSteps + 1];
   __shared__ float longest_w[kPlanWarps][kSimtSteps + 1];
-  __shared__ long long work[kSimtSteps + 1];
-  __shared__ float longest[kSimtSteps + 1];
+  __shared__ float makespan[kSimtSteps + 1];
+  __shared__ float longest;
   __shared__ float limit;
   pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the warps stand side by side over the matrices, as often as they go (each
+  // such group takes every groups-th step)
+  const int span = min((batch + 31) / 32, kPlanWarps);
+  const int group = warp / span, groups = kPlanWarps / span;
+  const int first = (warp - group * span) * 32 + lane;
+  const bool once = batch <= kPlanThreads;
+  int M = 0, N = 0, K = 0;  // the thread's matrix
+  bool any = false;
+  SimtCands e;
+  auto fetch = [&](int i) {
+    M = i < batch ? dM[i] : 0;
+    N = i < batch ? dN[i] : 0;
+    K = i < batch ? dK[i] : 0;
+    any = !fw_bad(M, N, K, max_dim) && M > 0 && N > 0;
+    if (any) simt_cands(M, N, K, -1, &e);
+  };
+  if (once && group < groups) fetch(first);
   if (threadIdx.x < kBins) bin_tiles[threadIdx.x] = 0;
   if (lane <= kSimtSteps) {
     work_w[warp][lane] = 0;
     longest_w[warp][lane] = 0.0f;
   }
   __syncwarp();
-  // steps from .. to, each warp's part
   auto sums = [&](int from, int to) {
-    for (int i0 = warp * 32; i0 < batch; i0 += kPlanThreads) {
-      const int i = i0 + lane;
-      const int M = i < batch ? dM[i] : 0, N = i < batch ? dN[i] : 0, K = i < batch ? dK[i] : 0;
-      const bool any = !fw_bad(M, N, K, max_dim) && M > 0 && N > 0;
-      SimtCands e;
-      if (any) simt_cands(M, N, K, -1, c_cfgs, c_cost, &e);
-      float T = from == 0 ? 3e38f : longest[0];
-      for (int j = from; j <= to; ++j) {
-        if (j > 0) T *= 0.70710678f;
-        float w = 0.0f, l = 0.0f;
-        if (any && simt_pick(e, T, &w, &l) < 0) w = l = 0.0f;
-        long long v = (long long)w;
-        for (int o = 16; o; o >>= 1) {
-          v += __shfl_xor_sync(0xffffffffu, v, o);
-          l = fmaxf(l, __shfl_xor_sync(0xffffffffu, l, o));
-        }
-        if (lane == 0) {
-          work_w[warp][j] += v;
-          longest_w[warp][j] = fmaxf(longest_w[warp][j], l);
+    if (group < groups) {
+      for (int i0 = first; i0 - lane < batch; i0 += span * 32) {
+        if (!once) fetch(i0);
+        float T = from == 0 ? 3e38f : simt_limit(longest, from + group);
+        for (int j = from + group; j <= to; j += groups) {
+          float w = 0.0f, l = 0.0f;
+          if (any && simt_pick(e, T, &w, &l) < 0) w = l = 0.0f;
+          const long long v = warp_sum((long long)w);
+          // (no time is negative: ordered as their bits are)
+          l = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(l)));
+          if (lane == 0) {
+            work_w[warp][j] += v;
+            longest_w[warp][j] = fmaxf(longest_w[warp][j], l);
+          }
+          T = simt_limit(T, groups);
         }
       }
     }
     __syncthreads();
-    if (threadIdx.x >= from && threadIdx.x <= to) {
-      long long v = 0;
-      float l = 0.0f;
-#pragma unroll 8
-      for (int w = 0; w < kPlanWarps; ++w) {
-        v += work_w[w][threadIdx.x];
-        l = fmaxf(l, longest_w[w][threadIdx.x]);
+    if (warp >= from && warp <= to) {  // step `warp`, every warp's part
+      const long long v = warp_sum(work_w[lane][warp]);
+      const float l = __uint_as_float(
+          __reduce_max_sync(0xffffffffu, __float_as_uint(longest_w[lane][warp])));
+      if (lane == 0) {
+        if (warp == 0) longest = l;
+        makespan[warp] = simt_makespan(v, l, slots);
       }
-      work[threadIdx.x] = v;
-      longest[threadIdx.x] = l;
     }
     __syncthreads();
   };
   sums(0, 0);
   sums(1, kSimtSteps);
-  if (threadIdx.x == 0) limit = simt_choose_limit(work, longest, slots);
+  if (threadIdx.x == 0) limit = simt_choose_limit(makespan, longest);
   __syncthreads();
   // each matrix reserves its tiles in the bin of its tile time
-  for (int i = threadIdx.x; i < batch; i += blockDim.x) {
-    const int M = dM[i], N = dN[i], K = dK[i];
+  int start = -1, bin = 0;
+  auto reserve = [&](int i) {
     MatDesc d{M, N, K, max(M, 1), max(K, 1), max(M, 1), 0, 0};
-    int start = -1;
+    start = -1;
     if (fw_bad(M, N, K, max_dim)) {
       atomicOr(s.err, 1);
-    } else if (M > 0 && N > 0) {
-      SimtCands e;
+    } else if (any) {
       float w, l;
-      simt_cands(M, N, K, -1, c_cfgs, c_cost, &e);
       const int c = simt_pick(e, limit, &w, &l);
       if (c >= 0) {
         d.cfg = c;
-        d.aux = fw_bin(K, c_cost[c]);
-        start = atomicAdd(&bin_tiles[d.aux], (int)simt_tiles(M, N, c_cfgs[c]));
+        d.aux = bin = fw_bin(K, c_cost[c]);
+        start = atomicAdd(&bin_tiles[bin], (int)simt_tiles(M, N, c_cfgs[c]));
       }
     }
     s.descs[i] = d;
-    s.mat_start[i] = start;
+  };
+  if (once) {
+    if (group == 0 && first < batch) reserve(first);
+  } else {
+    for (int i = threadIdx.x; i < batch; i += kPlanThreads) {
+      fetch(i);
+      reserve(i);
+      s.mat_start[i] = start;
+    }
   }
   __syncthreads();
   if (threadIdx.x < kBins) {  // longest tiles first
@@ -147,9 +178,13 @@ __global__ void __launch_bounds__(kPlanThreads)
     if (threadIdx.x == 0) *s.n_items = run + bin_tiles[0];
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < batch; i += blockDim.x) {
-    const int off = s.mat_start[i];
-    if (off >= 0) s.mat_start[i] = bin_start[s.descs[i].aux] + off;
+  if (once) {
+    if (group == 0 && first < batch) s.mat_start[first] = start < 0 ? -1 : bin_start[bin] + start;
+  } else {
+    for (int i = threadIdx.x; i < batch; i += kPlanThreads) {
+      const int off = s.mat_start[i];
+      if (off >= 0) s.mat_start[i] = bin_start[s.descs[i].aux] + off;
+    }
   }
 }
 
@@ -370,7 +405,7 @@ extern "C" int bgemm_debug_framework_plan(const int* M, const int* N, const int*
   auto any = [&](int i) { return !fw_bad(M[i], N[i], K[i], max_dim) && M[i] > 0 && N[i] > 0; };
   for (int i = 0; i < batch; ++i) {
     if (fw_bad(M[i], N[i], K[i], max_dim)) *err |= 1;
-    if (any(i)) simt_cands(M[i], N[i], K[i], -1, kSimtCfgs, kSimtCost, &cand[i]);
+    if (any(i)) simt_cands(M[i], N[i], K[i], -1, &cand[i]);
   }
   for (int j = 0; j <= kSimtSteps; ++j)
     for (int i = 0; i < batch; ++i) {

@@ -105,7 +105,7 @@ static bgemm_status_t choose_simt(const int* M, const int* N, const int* K, int 
   cur_l.resize((size_t)batch);
   for (int i = 0; i < batch; ++i) {
     if (M[i] == 0 || N[i] == 0) continue;
-    simt_cands(M[i], N[i], K[i], force, kSimtCfgs, kSimtCost, &cand[i]);
+    simt_cands(M[i], N[i], K[i], force, &cand[i]);
     if (simt_pick(cand[i], 3e38f, &cur_w[i], &cur_l[i]) < 0)
       return set_error(BGEMM_ERROR_NOT_SUPPORTED, 1, i, "matrix %d: no tile configuration fits",
                        i);

@@ -12,6 +12,8 @@
 #pragma once
 #include <math.h>
 
+#include <utility>
+
 #include "bgemm_internal.h"
 
 namespace bgemm {
@@ -89,8 +91,7 @@ constexpr int kTcCPrefetchLead = 0;
 // ------------------------------------------------- SIMT planning model --
 // Shared by the host planner, the device planner and its host replay, which
 // decide alike: single precision with explicit fmaf, work summed as whole
-// nanoseconds.  `cfgs` and `cost` are kSimtCfgs and kSimtCost, or the device's
-// copies of them.
+// nanoseconds.
 //
 // For each matrix the configuration with the least work (modelled time on the
 // CTAs) among those whose single tile takes no longer than a limit T, with T
@@ -135,16 +136,23 @@ __host__ __device__ inline float simt_work_ns(int M, int N, int K, SimtCfg g, Ti
 struct SimtCands {
   float work[kSimtNumCfgs], lat[kSimtNumCfgs];
 };
-__host__ __device__ inline void simt_cands(int M, int N, int K, int force, const SimtCfg* cfgs,
-                                           const TileCost* cost, SimtCands* e) {
-#pragma unroll
-  for (int c = 0; c < kSimtNumCfgs; ++c) {
-    e->work[c] = 0.0f;
-    e->lat[c] = -1.0f;
-    if ((force >= 0 ? c != force : !simt_auto_cfg(c, M, N)) || !simt_fits(M, N, cfgs[c])) continue;
-    e->work[c] = simt_work_ns(M, N, K, cfgs[c], cost[c]);
-    e->lat[c] = simt_alone_ns(K, cost[c], c);
-  }
+template <int C>
+__host__ __device__ inline void simt_cand(int M, int N, int K, int force, SimtCands* e) {
+  constexpr SimtCfg g = kSimtCfgs[C];
+  constexpr TileCost t = kSimtCost[C];
+  e->work[C] = 0.0f;
+  e->lat[C] = -1.0f;
+  if ((force >= 0 ? C != force : !simt_auto_cfg(C, M, N)) || !simt_fits(M, N, g)) return;
+  e->work[C] = simt_work_ns(M, N, K, g, t);
+  e->lat[C] = simt_alone_ns(K, t, C);
+}
+template <int... C>
+__host__ __device__ inline void simt_cands_of(std::integer_sequence<int, C...>, int M, int N,
+                                              int K, int force, SimtCands* e) {
+  (simt_cand<C>(M, N, K, force, e), ...);
+}
+__host__ __device__ inline void simt_cands(int M, int N, int K, int force, SimtCands* e) {
+  simt_cands_of(std::make_integer_sequence<int, kSimtNumCfgs>{}, M, N, K, force, e);
 }
 // Least work with a tile of at most T, or else the shortest tile (-1: none).
 __host__ __device__ inline int simt_pick(const SimtCands& e, float T, float* work, float* lat) {
@@ -168,26 +176,34 @@ __host__ __device__ inline int simt_pick(const SimtCands& e, float T, float* wor
   *lat = best >= 0 ? bl : sl;
   return best >= 0 ? best : any;
 }
-// T from the sums of every step (step 0: no limit; step j: the limit
-// simt_limit(longest[0], j)).
+// The limit of step j > 0, from the longest tile of step 0 (which has none).
 __host__ __device__ inline float simt_limit(float longest, int step) {
   float t = longest;
   for (int j = 0; j < step; ++j) t *= 0.70710678f;
   return t;
 }
-__host__ __device__ inline float simt_choose_limit(const long long* work, const float* longest,
-                                                   int slots) {
-  float best = 0.0f, limit = longest[0], T = 3e38f;  // limit: step j - 1's
+// The modelled makespan of a step on `slots` CTAs from its sums, and T from
+// every step's.
+__host__ __device__ inline float simt_makespan(long long work, float longest, int slots) {
+  return fmaf(kSimtTail, longest, (float)work / (float)slots);
+}
+__host__ __device__ inline float simt_choose_limit(const float* makespan, float longest) {
+  float best = 0.0f, limit = longest, T = 3e38f;  // limit: step j - 1's
   for (int j = 0; j <= kSimtSteps; ++j) {
     if (j > 0 && kSimtTail * limit <= 0.02f * best) break;
     if (j > 0) limit *= 0.70710678f;
-    const float m = fmaf(kSimtTail, longest[j], (float)work[j] / (float)slots);
-    if (j == 0 || m < best) {
-      best = m;
+    if (j == 0 || makespan[j] < best) {
+      best = makespan[j];
       T = j == 0 ? 3e38f : limit;
     }
   }
   return T;
+}
+
+inline float simt_choose_limit(const long long* work, const float* longest, int slots) {
+  float makespan[kSimtSteps + 1];
+  for (int j = 0; j <= kSimtSteps; ++j) makespan[j] = simt_makespan(work[j], longest[j], slots);
+  return simt_choose_limit(makespan, longest[0]);
 }
 
 }  // namespace bgemm
