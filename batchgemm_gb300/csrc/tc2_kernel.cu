@@ -57,6 +57,9 @@ constexpr int kSched = 4;                  // schedule slots (items published ah
 // contiguous in memory and [row][32] where k is.
 constexpr int kPackWarps = 2, kPackBufs = 4, kPackK2 = 32;
 constexpr int kPackFloats = kPackK2 * 33;
+// K from which a strip with contiguous k is walked in chunks of 8 rows x 128 k
+// instead of 32 x 32.
+constexpr int kPackWideK = 256;
 constexpr int kPackBytes = kPackFloats * 4;
 // Stage ring of 3 stages of 64 KB, two parts per side: the split modes' hi and
 // lo halves of one 128-byte K slice, or two consecutive K slices of the
@@ -127,10 +130,13 @@ __device__ __forceinline__ void cp16(uint32_t dst, const float* src, int bytes) 
 // proxy fence: the readers are TMA loads.
 // Bound by the issue of one warp: alone on the chip the 304 of them split the
 // skewed batch's 5.5 GB of operands in 3.5 ms (4.2 ms before inner chunks lost
-// their bounds), beside the GEMM in 5.7.  The copies also cost the GEMM: they
-// fill shared memory by 32-byte wavefronts beside the MMAs' operand reads.
-// Skewed batch, pre-pass then GEMM 9.45 ms, this way 8.6 to 9.0; a limit on how
-// far packing runs ahead of the tiles (one to eight waves) changed nothing.
+// their bounds), beside the GEMM in 5.7.  What it costs the GEMM is the packed
+// stores: half of it their way into L2, half their way on to HBM, from where
+// the GEMM reads them back (the operands in use at a time are larger than L2);
+// the copies into shared memory cost little.  Skewed batch, pre-pass then GEMM
+// 9.45 ms, this way 8.6 to 8.9; a limit on how far packing runs ahead of the
+// tiles (one to eight waves), stores that bypass a cache and L2 prefetch by the
+// producers changed nothing or made it slower.
 template <int KIND, int SPLIT>
 __device__ __forceinline__ void pack_strips(const TcGemmParams& p, float* buf, int lane,
                                             volatile int* abort) {
@@ -156,11 +162,44 @@ __device__ __forceinline__ void pack_strips(const TcGemmParams& p, float* buf, i
     const float* X = is_a ? p.A[job.mat] : p.B[job.mat];
     X += rows_contig ? (long long)job.r0 : (long long)job.r0 * ld;
     const bool vec = ((reinterpret_cast<uintptr_t>(X) & 15u) == 0) && (ld & 3) == 0;
+    // A chunk: 32 rows of 32 k or, where k is contiguous and long, 8 rows of
+    // 128 k.  The packed stores are what packing costs the GEMM (skewed batch
+    // 8.6 ms, 6.8 without them, 6.5 without packing at all), and rows of 256 or
+    // 512 bytes cost less than pieces of 64 or 128: row-major NT of 96 matrices
+    // of 97 to 1501 in BF16 521 -> 507 us, the skewed batch 9.00 -> 8.92 ms.
+    // Lines at K = 128 or 512: row 504 and 508 us, the skewed batch 0.3 and 0.8
+    // % slower than at 256.  The single product keeps the 32 x 32 chunks: its
+    // batch of 128 took 1280 us where this takes 1220 (registers).
+    const bool wide = SPLIT && !rows_contig && K >= kPackWideK;
+    const int kc = wide ? 128 : kPackK2, rc = wide ? 8 : 32;
+    const int rows_end = K > 0 ? min(rows, 32) : 0;
     // one chunk's copies; inner ones carry no bounds
-    auto load = [&](int k0, float* s) {
+    auto load = [&](int k0, int r, float* s) {
       const uint32_t dst = smem_u32(s) + lane * 4;
       const int ks = K - k0;
-      if (rows_contig) {
+      if (wide) {
+        const float* src = X + (long long)r * ld + k0;
+        if (vec) {
+          const int bytes = min(max(ks - 4 * lane, 0), 4) * 4;
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            cp16(dst + (i * 128 + 3 * lane) * 4, src + (long long)ld * i + 4 * lane,
+                 r + i < rows ? bytes : 0);
+        } else if (ks >= 128 && r + 8 <= rows) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              cp4(dst + (i * 128 + q * 32) * 4, src + (long long)ld * i + q * 32 + lane, 4);
+        } else {
+#pragma unroll 1
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              cp4(dst + (i * 128 + q * 32) * 4, src + (long long)ld * i + q * 32 + lane,
+                  r + i < rows && q * 32 + lane < ks ? 4 : 0);
+        }
+      } else if (rows_contig) {
         const float* src = X + (long long)k0 * ld + lane;
         const int bytes = lane < rows ? 4 : 0;
         if (ks >= kPackK2) {
@@ -196,29 +235,39 @@ __device__ __forceinline__ void pack_strips(const TcGemmParams& p, float* buf, i
     const PackDesc* pd = p.pdescs + job.mat;
     const int kpad = pd->kpad;
     constexpr int E = KIND == kKindTF32 ? 4 : 2;  // bytes of a packed element
-    // eight lanes to a packed row, four k each; four rows at a time
-    const int r4 = lane >> 3, kq = (lane & 7) * 4;
-    const long long at0 = (long long)(job.r0 + r4) * kpad + kq;
-    char* hi = p.ws + (is_a ? pd->a_hi : pd->b_hi) + at0 * E;
-    char* lo = p.ws + (is_a ? pd->a_lo : pd->b_lo) + at0 * E;
-    const long long step = 4ll * kpad;  // elements
-#pragma unroll 1
-    for (int c = 0; c < kPackBufs - 1; ++c) {
-      if (c * kPackK2 < K)
-        load(c * kPackK2, buf + c * kPackFloats);
-      else
+    // four k a lane: eight lanes to a packed row and four rows at a time, or
+    // the warp to a row
+    const int r4 = wide ? 0 : lane >> 3, kq = (wide ? lane : lane & 7) * 4;
+    const int rstep = wide ? 1 : 4;
+    const long long step = (long long)rstep * kpad;  // elements
+    char* const hi0 = p.ws + (is_a ? pd->a_hi : pd->b_hi);
+    char* const lo0 = p.ws + (is_a ? pd->a_lo : pd->b_lo);
+    int lk = 0, lr = 0;  // the next chunk to load
+    auto load_next = [&](int b) {
+      if (lr < rows_end) {
+        load(lk, lr, buf + b * kPackFloats);
+        lk += kc;
+        if (lk >= K) {
+          lk = 0;
+          lr += rc;
+        }
+      } else {
         asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    int rd = 0, wr = kPackBufs - 1;
+      }
+    };
 #pragma unroll 1
-    for (int k0 = 0; k0 < K; k0 += kPackK2) {
+    for (int c = 0; c < kPackBufs - 1; ++c) load_next(c);
+    int rd = 0, wr = kPackBufs - 1, k0 = 0, r0 = 0;
+#pragma unroll 1
+    while (r0 < rows_end) {
       asm volatile("cp.async.wait_group %0;" ::"n"(kPackBufs - 2) : "memory");
       __syncwarp();  // (and every lane is done with the buffer that is filled next)
-      if (k0 + (kPackBufs - 1) * kPackK2 < K)
-        load(k0 + (kPackBufs - 1) * kPackK2, buf + wr * kPackFloats);
-      else
-        asm volatile("cp.async.commit_group;" ::: "memory");
-      const float* s = buf + rd * kPackFloats + (rows_contig ? kq * 33 + r4 : r4 * kPackK2 + kq);
+      load_next(wr);
+      const long long at = (long long)(job.r0 + r0 + r4) * kpad + k0 + kq;
+      char* hi = hi0 + at * E;
+      char* lo = lo0 + at * E;
+      // (k contiguous: r4 * 32 + kq, or kq, are 4 * lane in either form)
+      const float* s = buf + rd * kPackFloats + (rows_contig ? kq * 33 + r4 : 4 * lane);
       auto fetch = [&](int it, float(&x)[4]) {
         if (rows_contig) {
 #pragma unroll
@@ -228,7 +277,7 @@ __device__ __forceinline__ void pack_strips(const TcGemmParams& p, float* buf, i
           x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
         }
       };
-      if (rows >= 32 && k0 + kPackK2 <= K) {
+      if (rows - r0 >= rc && k0 + kc <= K) {
         // (four rows of fragments at a time, for their latencies to overlap)
 #pragma unroll
         for (int i0 = 0; i0 < 8; i0 += 4) {
@@ -242,7 +291,7 @@ __device__ __forceinline__ void pack_strips(const TcGemmParams& p, float* buf, i
 #pragma unroll 1
         for (int it = 0; it < 8; ++it) {
           const int left = K - k0 - kq;
-          if (it * 4 + r4 < rows && left > 0) {
+          if (r0 + it * rstep + r4 < rows && left > 0) {
             float x[4];
             fetch(it, x);
             if (left >= 4) {
@@ -255,8 +304,11 @@ __device__ __forceinline__ void pack_strips(const TcGemmParams& p, float* buf, i
           }
         }
       }
-      hi += kPackK2 * E;
-      lo += kPackK2 * E;
+      k0 += kc;
+      if (k0 >= K) {
+        k0 = 0;
+        r0 += rc;
+      }
       rd = rd + 1 == kPackBufs ? 0 : rd + 1;
       wr = wr + 1 == kPackBufs ? 0 : wr + 1;
     }
