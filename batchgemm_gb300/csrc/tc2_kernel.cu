@@ -83,10 +83,11 @@ constexpr int kCols = 128;                 // accumulator columns per epilogue w
 // two packing warps; warpgroups 1 and 2 = the 8 epilogue warps.  At launch every
 // thread gets 168 registers (3 warps per SM sub-partition); warpgroup 0 gives
 // most of its share to the epilogue warps, whose 128 accumulator columns per
-// lane would otherwise spill: 128 x 56 + 256 x 224 = 384 x 168.
+// lane would otherwise spill: 128 x 72 + 256 x 216 = 384 x 168.  (At 56 and
+// 224 the packing warps spilled: batch stream 6846 us, 6812 this way.)
 constexpr int kThreads2 = 384;
 constexpr int kEpiWarp0 = 4;               // first epilogue warp
-constexpr uint32_t kRegsCtl = 56, kRegsEpi = 224, kRegsLaunch = 168;
+constexpr uint32_t kRegsCtl = 72, kRegsEpi = 216, kRegsLaunch = 168;
 static_assert(128 * kRegsCtl + 256 * kRegsEpi <= kThreads2 * kRegsLaunch, "register split");
 // Promotion groups of the split modes come per bucket of K from the launch's
 // TcSchedule (autotuned table): group g > 0 = g 128-byte K slices per TMEM
@@ -168,8 +169,8 @@ __device__ __forceinline__ void pack_strips(const TcGemmParams& p, float* buf, i
     // 512 bytes cost less than pieces of 64 or 128: row-major NT of 96 matrices
     // of 97 to 1501 in BF16 521 -> 507 us, the skewed batch 9.00 -> 8.92 ms.
     // Lines at K = 128 or 512: row 504 and 508 us, the skewed batch 0.3 and 0.8
-    // % slower than at 256.  The single product keeps the 32 x 32 chunks: its
-    // batch of 128 took 1280 us where this takes 1220 (registers).
+    // % slower than at 256.  The single product keeps the 32 x 32 chunks: no
+    // faster with the others (1227 and 1224 us, 128 matrices of N = K = 1024).
     const bool wide = SPLIT && !rows_contig && K >= kPackWideK;
     const int kc = wide ? 128 : kPackK2, rc = wide ? 8 : 32;
     const int rows_end = K > 0 ? min(rows, 32) : 0;
