@@ -1,8 +1,9 @@
 // tc_kernel.cu -- tensor-core (tcgen05 / TMEM) form of the variable-size
 // batched SGEMM for sm_103a.
 //
-// Two kernels per execute:
-//   tc_pack_kernel  splits every operand element x into hi = round(x) and
+// Kernels:
+//   tc_pack_kernel  (before the GEMM below, whole; before the CTA-pair GEMM,
+//                   tc2_kernel.cu, the operands of the first tiles) splits every operand element x into hi = round(x) and
 //                   lo = round(x - hi) (TF32 or BF16, round to nearest even)
 //                   and writes them K-major ("rows of K", 16-byte aligned row
 //                   length) into the plan's workspace: A is transposed from
