@@ -102,9 +102,14 @@ constexpr float kSimtTail = 1.0f;     // share of the longest tile that is not h
 constexpr float kSimtFma = 0.35f;     // time per k that a skipped edge saves
 constexpr int kSimtSteps = 12;
 
-// (bm, bn, gm and gn are powers of two)
-__host__ __device__ inline int simt_tiles_m(int M, SimtCfg g) { return (M + g.bm - 1) >> g.lm; }
-__host__ __device__ inline int simt_tiles_n(int N, SimtCfg g) { return (N + g.bn - 1) >> g.ln; }
+// (bm, bn, gm and gn are powers of two; unsigned, since sizes go up to the
+// largest int and simt_fits has to refuse those)
+__host__ __device__ inline int simt_tiles_m(int M, SimtCfg g) {
+  return (int)(((unsigned)M + (unsigned)(g.bm - 1)) >> g.lm);
+}
+__host__ __device__ inline int simt_tiles_n(int N, SimtCfg g) {
+  return (int)(((unsigned)N + (unsigned)(g.bn - 1)) >> g.ln);
+}
 __host__ __device__ inline bool simt_fits(int M, int N, SimtCfg g) {
   // TileItem holds 16-bit tile coordinates
   return simt_tiles_m(M, g) <= 65535 && simt_tiles_n(N, g) <= 65535;
