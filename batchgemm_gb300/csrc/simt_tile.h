@@ -636,6 +636,8 @@ __device__ __forceinline__ void persistent_body(const SimtParams& p) {
         }
         if (cfg == 0) {
           next = run_tile<Shape<1, 1, 4, 4, 2, TA, TB>>(p, ti.mat, ti.tm * 16, ti.tn * 16, true);
+          // the staged C has been read: the next tile's copies may land there
+          __syncwarp();
         } else {
           // ids 1 to 6: 32 x 32 parts in turn (1 x 1, 2 x 1, 1 x 2, ...); the
           // first is inside the matrix, the last may not be
