@@ -8,12 +8,13 @@
 // a CTA.  A warp's lanes form an LX x LY grid and each thread owns TM x TN
 // outputs.  The thin tiles (8 x 128, 128 x 8) are bound by the bytes they read
 // for a few FMAs each: all eight warps share one tile's long operand, in
-// slices of 32 k, so that a CTA keeps 55 KB on the way and a long K ends soon.
+// slices of 32 k, so that a CTA keeps 55 KB on the way and a long K ends soon
+// (run_thin).
 // Operands stream through a cp.async ring of BK k-slices:
 //   A slice: [k][BM]      rows contiguous, 16-byte cp.async when lda % 4 == 0
 //                         and A is 16-byte aligned, 4-byte otherwise
 //   B slice: [n][BK + 4]  k contiguous, as B is stored: 16-byte cp.async on
-//                         the same condition; rows of BK + 4 floats (12 or 20)
+//                         the same condition; rows of BK + 4 floats (20 or 36)
 //                         put the float4 reads of eight lanes on distinct banks
 //                         (the 128 x 128 tile: [k][BN + 4])
 // An operand stored the other way round from its slice (A as K x M) is
@@ -104,16 +105,20 @@ __device__ __forceinline__ int thread_index() {
 }
 
 // Tile shape, ring geometry and index maps of a team of WM x WN warps, each of
-// LX x (32 / LX) lanes.  TA / TB: A stored K x M, B stored N x K.
-template <int WM_, int WN_, int LX_, int TM_, int TN_, bool TA_, bool TB_, int BK_ = 0>
+// LX x (32 / LX) lanes.  TA / TB: A stored K x M, B stored N x K.  CT: the tile
+// is computed as C^T = B^T A^T, that is, all of the below is said of B^T, A^T
+// and C^T.  SHIFT: B's slice holds each row from the 16-byte boundary before it.
+template <int WM_, int WN_, int LX_, int TM_, int TN_, bool TA_, bool TB_, int BK_ = 0,
+          bool CT_ = false, bool SHIFT_ = false>
 struct Shape {
   static constexpr int WM = WM_, WN = WN_, LX = LX_, TM = TM_, TN = TN_;
-  static constexpr bool TA = TA_, TB = TB_;
+  static constexpr bool TA = TA_, TB = TB_, CT = CT_, SHIFT = SHIFT_;
   static constexpr int NT = 32 * WM * WN, LY = 32 / LX;
   static constexpr int WBM = LX * TM, WBN = LY * TN;  // a warp's part of the tile
   static constexpr int BM = WM * WBM, BN = WN * WBN;
   static_assert(NT == 32 || NT == kThreads, "a team is a warp or the CTA");
   static_assert(TM % 4 == 0 && (TN % 4 == 0 || TN <= 2), "register tile");
+  static_assert(!SHIFT || (TN == 1 && !TB), "one offset per thread");
   static constexpr int kBudget = NT == 32 ? kWarpFloats : kWarps * kWarpFloats;
   // B's slice by rows of n (else of k): as an N x K operand is stored, and
   // wherever 64 accumulators leave no registers for fragments of several k
@@ -135,6 +140,9 @@ struct Shape {
   }
   static constexpr int NS = fit(kSimtRingCap);
   static_assert(NS >= 2 && STAGE % 4 == 0 && A_STAGE % 4 == 0, "ring geometry");
+  // (fragments are read up to one k behind a slice)
+  static_assert((NS - 1) * STAGE + A_STAGE + LDA <= kBudget && NS * STAGE + LDB <= kBudget,
+                "reads ahead");
 
   // A lane's place in the grid: eight consecutive lanes take 4 x 2 places, so
   // that a 16-byte fragment read moves 64 and 32 distinct bytes per quarter
@@ -217,7 +225,8 @@ __device__ __forceinline__ void load_rows_contig(const float* X, int ldx, int ro
     const uint32_t dst = smem_u32(s + kk0 * LDS + rr);
     if (BK % KS == 0 || kk0 < BK)
       copies<16, (BK + KS - 1) / KS, KS, KS * LDS * 4, KS>(dst, src, ldx, valid, ks - kk0, full);
-  } else if constexpr (NT >= R) {
+  } else {
+    static_assert(NT >= R, "one row position per thread");
     constexpr int KS = NT / R;
     const int rr = tid % R, kk0 = tid / R;
     const float* src = X + (long long)kk0 * ldx + rr;
@@ -225,10 +234,6 @@ __device__ __forceinline__ void load_rows_contig(const float* X, int ldx, int ro
     if (BK % KS == 0 || kk0 < BK)
       copies<4, (BK + KS - 1) / KS, KS, KS * LDS * 4, KS>(dst, src, ldx, rr < rows ? 4 : 0,
                                                           ks - kk0, full);
-  } else {
-#pragma unroll 1
-    for (int rr = tid; rr < R; rr += NT)
-      copies<4, BK, 1, LDS * 4, 1>(smem_u32(s + rr), X + rr, ldx, rr < rows ? 4 : 0, ks, full);
   }
 }
 
@@ -259,6 +264,43 @@ __device__ __forceinline__ void load_k_contig(const float* X, int ldx, int rows,
   }
 }
 
+// Floats from the 16-byte boundary at or before X to X.
+__device__ __forceinline__ int floats_off(const float* X) {
+  return (int)(reinterpret_cast<uintptr_t>(X) >> 2) & 3;
+}
+// The same slices, k contiguous, rows that start anywhere: 16-byte copies from
+// the boundary at or before each row's k on, so that s[r][LDS] holds the slice
+// from float floats_off(row) on.  What lies before the row's first element
+// (`first`: the slices start there) and behind its last is not read.
+template <int NT, int R, int LDS, int BK>
+__device__ __forceinline__ void load_k_shifted(const float* X, int ldx, int rows, int ks, float* s,
+                                               bool first, int tid) {
+  constexpr int KC = BK / 4, RS = NT / KC;  // chunks of a row, the last one apart
+  static_assert(LDS >= BK + 4 && R % RS == 0 && RS % 4 == 0 && R <= NT, "chunks");
+  const int c = tid % KC, rr0 = tid / KC;
+  const float* row = X + (long long)rr0 * ldx;
+  const int off = floats_off(row);  // that of every RS-th row
+  const uint32_t dst = smem_u32(s + rr0 * LDS + c * 4);
+  if (first && c == 0 && off > 0) {
+#pragma unroll 1
+    for (int r = 0; r < R; r += RS)
+      for (int q = off; q < 4; ++q)
+        cp_async4(dst + (r * LDS + q) * 4, row + (long long)r * ldx + (q - off),
+                  rr0 + r < rows && q - off < ks ? 4 : 0);
+  } else {
+    copies<16, R / RS, RS, RS * LDS * 4, RS>(dst, row - off + c * 4, ldx,
+                                             min(max(ks + off - c * 4, 0), 4) * 4, rows - rr0,
+                                             rows >= R);
+  }
+  if (tid < R) {
+    const float* last = X + (long long)tid * ldx;
+    const int o = floats_off(last);
+    if (o > 0)
+      cp_async16(smem_u32(s + tid * LDS + BK), last - o + BK,
+                 tid < rows ? min(max(ks + o - BK, 0), 4) * 4 : 0);
+  }
+}
+
 // One k of the register tile's first HM * 4 rows and NJ columns: the row pair
 // stays the operand of NJ FMAs in a row and the columns run back and forth, so
 // that consecutive FMAs share register operands (measured on FFMA2 alone,
@@ -280,12 +322,12 @@ __device__ __forceinline__ void fma_tile(const f32x2 (&a)[TM / 2], const float (
 
 // acc += A slice * B slice, k in order, for the first HM of the TM / 4 row
 // groups and NJ of the TN columns a thread owns; sA and sB are at the thread's
-// first row and column.
+// first row and column (SHIFT: sB at the boundary `off` floats before it).
 template <class S, int HM, int NJ>
-__device__ __forceinline__ void compute_part(const float* sA, const float* sB, int ks,
+__device__ __forceinline__ void compute_part(const float* sA, const float* sB, int off, int ks,
                                              f32x2 (&acc)[S::TM / 2][S::TN]) {
   constexpr int TM = S::TM, TN = S::TN;
-  // long slices (the thin tiles') end with the matrix's K, rounded up to 4
+  // long slices end with the matrix's K, rounded up to 4
   constexpr bool kLong = S::BK > 16;
   const int k_end = kLong ? min(S::BK, (ks + 3) & ~3) : S::BK;
   auto load_a = [&](int k, f32x2(&a)[TM / 2]) {
@@ -299,13 +341,27 @@ __device__ __forceinline__ void compute_part(const float* sA, const float* sB, i
   };
   constexpr int UN = kLong ? 2 : S::BK / 4;
   if constexpr (!S::BROWS) {
+    float4 ahead;
+    if constexpr (S::SHIFT) ahead = *reinterpret_cast<const float4*>(sB);
 #pragma unroll UN
     for (int kq = 0; kq < k_end; kq += 4) {
       float b[4][TN];
+      if constexpr (S::SHIFT) {
+        // eight floats in two aligned reads, the row's four by selects (four
+        // 4-byte reads of 16 lanes' rows would take eight wavefronts, not two)
+        const float4 u = ahead;
+        ahead = *reinterpret_cast<const float4*>(sB + kq + 4);
+        const bool two = (off & 2) != 0, one = (off & 1) != 0;
+        const float t0 = two ? u.z : u.x, t1 = two ? u.w : u.y, t2 = two ? ahead.x : u.z;
+        const float t3 = two ? ahead.y : u.w, t4 = two ? ahead.z : ahead.x;
+        b[0][0] = one ? t1 : t0; b[1][0] = one ? t2 : t1;
+        b[2][0] = one ? t3 : t2; b[3][0] = one ? t4 : t3;
+      } else {
 #pragma unroll
-      for (int j = 0; j < NJ; ++j) {
-        const float4 v = *reinterpret_cast<const float4*>(sB + j * S::LY * S::LDB + kq);
-        b[0][j] = v.x; b[1][j] = v.y; b[2][j] = v.z; b[3][j] = v.w;
+        for (int j = 0; j < NJ; ++j) {
+          const float4 v = *reinterpret_cast<const float4*>(sB + j * S::LY * S::LDB + kq);
+          b[0][j] = v.x; b[1][j] = v.y; b[2][j] = v.z; b[3][j] = v.w;
+        }
       }
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
@@ -350,42 +406,52 @@ __device__ __forceinline__ void compute_part(const float* sA, const float* sB, i
 // The part of the register tile that a ragged edge leaves: half the rows and
 // half the columns are skipped where they are all outside the matrix, and the
 // whole where nothing is inside (mrem and nrem: rows and columns left from the
-// warp's first on; ks: k left).  A skipped FMA's issue slots go to the SM's other warps.
+// warp's first on; ks: k left).  A skipped FMA's issue slots go to the SM's
+// other warps.
 template <class S>
-__device__ __forceinline__ void compute_stage(const float* sA, const float* sB, int mrem, int nrem,
-                                              int ks, f32x2 (&acc)[S::TM / 2][S::TN]) {
+__device__ __forceinline__ void compute_stage(const float* sA, const float* sB, int off, int mrem,
+                                              int nrem, int ks,
+                                              f32x2 (&acc)[S::TM / 2][S::TN]) {
   constexpr int HM = S::TM / 4, TN = S::TN;
   if (mrem <= 0 || nrem <= 0) return;
   const bool half_m = HM == 2 && mrem <= S::LX * 4;
   constexpr bool kHalfN = S::BROWS ? TN == 8 : TN >= 2;
   const bool half_n = kHalfN && nrem <= S::WBN / 2;
   if (!half_m && !half_n)
-    compute_part<S, HM, TN>(sA, sB, ks, acc);
+    compute_part<S, HM, TN>(sA, sB, off, ks, acc);
   else if (!half_m)
-    compute_part<S, HM, kHalfN ? TN / 2 : TN>(sA, sB, ks, acc);
+    compute_part<S, HM, kHalfN ? TN / 2 : TN>(sA, sB, off, ks, acc);
   else if (!half_n)
-    compute_part<S, 1, TN>(sA, sB, ks, acc);
+    compute_part<S, 1, TN>(sA, sB, off, ks, acc);
   else
-    compute_part<S, 1, kHalfN ? TN / 2 : TN>(sA, sB, ks, acc);
+    compute_part<S, 1, kHalfN ? TN / 2 : TN>(sA, sB, off, ks, acc);
 }
 
 // How a warp walks its part of C, lanes along consecutive rows: access e of E
 // covers CPI columns (parts of fewer than 32 rows) or a 32-row piece of one.
+// CT: lanes along consecutive columns of C^T, which are C's rows.
 template <class S>
 struct CWalk {
   static constexpr int CPI = S::WBM < 32 ? 32 / S::WBM : 1;
   static constexpr int RPC = S::WBM < 32 ? 1 : S::WBM / 32;
   static constexpr int E = S::WBN / CPI * RPC;
-  static_assert(S::WBN % CPI == 0 && E % 4 == 0, "C walk");
+  static_assert(S::WBN % CPI == 0 && E % 4 == 0 && (!S::CT || S::WBN < 32), "C walk");
   // aligned C: four rows per lane, CPI4 columns per access
   static constexpr int CPI4 = 128 / S::WBM, E4 = S::WBN / CPI4;
-  static_assert(S::WBN % CPI4 == 0, "C walk");
+  static_assert(S::CT || S::WBN % CPI4 == 0, "C walk");
   int lm, lc;
   __device__ __forceinline__ explicit CWalk(int lane)
-      : lm(S::WBM < 32 ? lane % S::WBM : lane), lc(S::WBM < 32 ? lane / S::WBM : 0) {}
-  __device__ __forceinline__ int m(int e) const { return lm + e % RPC * 32; }
-  __device__ __forceinline__ int n(int e) const { return e / RPC * CPI + lc; }
+      : lm(S::CT ? lane / S::WBN : S::WBM < 32 ? lane % S::WBM : lane),
+        lc(S::CT ? lane % S::WBN : S::WBM < 32 ? lane / S::WBM : 0) {}
+  __device__ __forceinline__ int m(int e) const {
+    return lm + (S::CT ? e * (32 / S::WBN) : e % RPC * 32);
+  }
+  __device__ __forceinline__ int n(int e) const { return S::CT ? lc : e / RPC * CPI + lc; }
 };
+template <class S>
+__device__ __forceinline__ long long c_at(const MatDesc& d, int m, int n) {
+  return S::CT ? (long long)m * d.ldc + n : (long long)n * d.ldc + m;
+}
 
 // The warp's part of C (first row and column m0, n0) into sC, zero outside the
 // matrix: asynchronous copies, all in flight together.
@@ -393,7 +459,7 @@ template <class S>
 __device__ __forceinline__ void fetch_c(const float* C, const MatDesc& d, int m0, int n0,
                                         float* sC, int lane) {
   using W = CWalk<S>;
-  if (vec16(C, d.ldc)) {
+  if (!S::CT && vec16(C, d.ldc)) {
     const int lm = lane % (32 / W::CPI4) * 4, lc = lane / (32 / W::CPI4);
     const int valid = min(max(d.M - m0 - lm, 0), 4) * 4;
 #pragma unroll 4
@@ -408,9 +474,17 @@ __device__ __forceinline__ void fetch_c(const float* C, const MatDesc& d, int m0
 #pragma unroll 4
   for (int e = 0; e < W::E; ++e) {
     const int m = m0 + w.m(e), n = n0 + w.n(e);
-    cp_async4(smem_u32(sC + w.n(e) * S::LDC + w.m(e)), C + (long long)n * d.ldc + m,
+    cp_async4(smem_u32(sC + w.n(e) * S::LDC + w.m(e)), C + c_at<S>(d, m, n),
               m < d.M && n < d.N ? 4 : 0);
   }
+}
+
+// Matrix `mat` of the queue (CT: of the transposed product).
+template <class S>
+__device__ __forceinline__ MatDesc desc_of(const SimtParams& p, int mat) {
+  const MatDesc d = p.descs[mat];
+  if constexpr (S::CT) return MatDesc{d.N, d.M, d.K, d.ldb, d.lda, d.ldc, d.cfg, d.aux};
+  return d;
 }
 
 __device__ __forceinline__ volatile int* control() {
@@ -426,9 +500,10 @@ constexpr int kNoItem = 0x7fffffff;
 // One tile of matrix `mat` whose first row and column are m0 and n0, by the
 // calling team.  With `pull` the team's first thread takes its next item while
 // C is written (the atomic's round trip is then hidden) and gets it back; a
-// warp takes none when another warp of the CTA waits with a CTA tile.  A real call: inlined beside one another the shapes spilled in
-// their k loops, by another amount after every edit (the 2048-matrix beta =
-// 0.5 batch took 2.77 ms with calls, 2.87 to 3.75 ms inlined).
+// warp takes none when another warp of the CTA waits with a CTA tile.  A real
+// call: inlined beside one another the shapes spilled in their k loops, by
+// another amount after every edit (the 2048-matrix beta = 0.5 batch took 2.77
+// ms with calls, 2.87 to 3.75 ms inlined).
 template <class S>
 __device__ __noinline__ int run_tile(const SimtParams& p, int mat, int m0, int n0, bool pull) {
   constexpr int TM = S::TM, TN = S::TN, NS = S::NS, BK = S::BK;
@@ -444,19 +519,22 @@ __device__ __noinline__ int run_tile(const SimtParams& p, int mat, int m0, int n
 
   f32x2 acc[TM / 2][TN];
   {
-    const MatDesc d = p.descs[mat];
-    const bool a_vec = vec16(p.A[mat], d.lda), b_vec = vec16(p.B[mat], d.ldb);
+    const MatDesc d = desc_of<S>(p, mat);
+    const float* A = S::CT ? p.B[mat] : p.A[mat];
+    const float* B = S::CT ? p.A[mat] : p.B[mat];
+    const bool a_vec = vec16(A, d.lda), b_vec = vec16(B, d.ldb);
     // the tile's first row and column at the k of the next stage to load
-    const float* A = p.A[mat] + (S::TA ? (long long)m0 * d.lda : (long long)m0);
-    const float* B = p.B[mat] + (S::TB ? (long long)n0 : (long long)n0 * d.ldb);
+    A += S::TA ? (long long)m0 * d.lda : (long long)m0;
+    B += S::TB ? (long long)n0 : (long long)n0 * d.ldb;
     const int mrem = d.M - m0, nrem = d.N - n0;
+    const int b_off = S::SHIFT ? floats_off(B + (long long)(wn + ly) * d.ldb) : 0;
 
     // alpha = beta = 1: the chains start from C, as the reference's do; its
     // old values come in behind the prologue's stages
     const bool inplace = p.alpha == 1.0f && p.beta == 1.0f;
     if (inplace) {
       fetch_c<S>(p.C[mat], d, m0 + wm, n0 + wn, sC, lane);
-    } else if (p.beta != 0.0f) {
+    } else if (!S::CT && p.beta != 0.0f) {
       const float* C = p.C[mat];
       for (int c = lane; c < S::WBN; c += 32) {
         const int n = n0 + wn + c, m = m0 + wm;
@@ -485,6 +563,8 @@ __device__ __noinline__ int run_tile(const SimtParams& p, int mat, int m0, int n
         load_rows_contig<S::NT, S::BM, S::LDA, BK>(A, lda, mrem, to_load, sA, a_vec, tid);
       if constexpr (S::TB)
         load_rows_contig<S::NT, S::BN, S::LDB, BK>(B, ldb, nrem, to_load, sB, b_vec, tid);
+      else if constexpr (S::SHIFT)
+        load_k_shifted<S::NT, S::BN, S::LDB, BK>(B, ldb, nrem, to_load, sB, to_load == d.K, tid);
       else
         load_k_contig<S::NT, S::BN, S::LDB, BK, S::BROWS>(B, ldb, nrem, to_load, sB, b_vec, tid);
       A += S::TA ? (long long)BK : (long long)BK * lda;
@@ -522,7 +602,7 @@ __device__ __noinline__ int run_tile(const SimtParams& p, int mat, int m0, int n
       const float* sA = ring + rd_slot * S::STAGE;
       compute_stage<S>(sA + wm + lx * 4,
                        sA + S::A_STAGE + (S::BROWS ? wn + S::n_of(ly, 0) : (wn + ly) * S::LDB),
-                       mrem - wm, nrem - wn, k_left, acc);
+                       b_off, mrem - wm, nrem - wn, k_left, acc);
       rd_slot = rd_slot + 1 == NS ? 0 : rd_slot + 1;
       wr_slot = wr_slot + 1 == NS ? 0 : wr_slot + 1;
     }
@@ -534,7 +614,7 @@ __device__ __noinline__ int run_tile(const SimtParams& p, int mat, int m0, int n
   // The outputs pass through shared memory, so that lanes walk consecutive
   // rows; old values of C come in there first.  The matrix is read again
   // instead of being held through the k loop.
-  const MatDesc d = p.descs[mat];
+  const MatDesc d = desc_of<S>(p, mat);
   float* C = p.C[mat];
   int next = kNoItem;
   if (pull && tid == 0 && (S::NT != 32 || control()[kCtlPosts] == 0)) next = pull_item(p);
@@ -567,7 +647,7 @@ __device__ __noinline__ int run_tile(const SimtParams& p, int mat, int m0, int n
     __syncwarp();
   }
   using W = CWalk<S>;
-  if (vec16(C, d.ldc)) {
+  if (!S::CT && vec16(C, d.ldc)) {
     const int lm = lane % (32 / W::CPI4) * 4, lc = lane / (32 / W::CPI4);
     const int m = m0 + wm + lm;
 #pragma unroll 4
@@ -591,9 +671,28 @@ __device__ __noinline__ int run_tile(const SimtParams& p, int mat, int m0, int n
 #pragma unroll 4
   for (int e = 0; e < W::E; ++e) {
     const int m = m0 + wm + w.m(e), n = n0 + wn + w.n(e);
-    if (m < d.M && n < d.N) C[(long long)n * d.ldc + m] = sC[w.n(e) * S::LDC + w.m(e)];
+    if (m < d.M && n < d.N) C[c_at<S>(d, m, n)] = sC[w.n(e) * S::LDC + w.m(e)];
   }
   return next;
+}
+
+// An 8 x 128 tile of A B (CT: of B^T A^T, a 128 x 8 tile of C).  The long
+// operand decides the form: where its k is contiguous it is staged as it lies,
+// each lane with a row of it; else as slices of k, each lane with four rows,
+// which is the 128 x 8 form of the transposed product.  Copies of 4 bytes pass
+// through the L1, of which two CTAs' shared memory leaves 26 KB: rows that
+// start anywhere take 16-byte copies from the boundary before them and selects
+// (600 matrices of 8 x 1024 x 512 at odd leading dimensions: 524 us with 4-byte
+// copies, 377 so; their transposes 600 and 376, on 16 bytes 467 and 297).
+template <bool TA, bool TB, bool CT>
+__device__ __forceinline__ int run_thin(const SimtParams& p, int mat, int m0, int n0, bool pull) {
+  if constexpr (TB) {
+    return run_tile<Shape<8, 1, 4, 4, 1, false, !TA, 32, !CT>>(p, mat, n0, m0, pull);
+  } else {
+    const bool vec = CT ? vec16(p.A[mat], p.descs[mat].lda) : vec16(p.B[mat], p.descs[mat].ldb);
+    return vec ? run_tile<Shape<1, 8, 2, 4, 1, TA, false, 32, CT>>(p, mat, m0, n0, pull)
+               : run_tile<Shape<1, 8, 2, 4, 1, TA, false, 32, CT, true>>(p, mat, m0, n0, pull);
+  }
 }
 
 // The persistent kernel's body.  CTAs pull items of the largest-first queue
@@ -667,9 +766,9 @@ __device__ __forceinline__ void persistent_body(const SimtParams& p) {
       const int cfg = p.descs[ti.mat].cfg;
       const bool pull = q == posts - 1 && n_items > (int)gridDim.x;
       if (cfg == 8)
-        next = run_tile<Shape<1, 8, 2, 4, 1, TA, TB, 32>>(p, ti.mat, ti.tm * 8, ti.tn * 128, pull);
+        next = run_thin<TA, TB, false>(p, ti.mat, ti.tm * 8, ti.tn * 128, pull);
       else if (cfg == 9)
-        next = run_tile<Shape<8, 1, 4, 4, 1, TA, TB, 32>>(p, ti.mat, ti.tm * 128, ti.tn * 8, pull);
+        next = run_thin<!TB, !TA, true>(p, ti.mat, ti.tn * 8, ti.tm * 128, pull);
       else
         next = run_tile<Shape<2, 4, 8, 8, 8, TA, TB>>(p, ti.mat, ti.tm * 128, ti.tn * 128, pull);
     }
