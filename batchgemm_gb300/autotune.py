@@ -90,7 +90,7 @@ def measure(mode, cfg, K, slots, waves=6, reps=5, hbm_gbs=6000.0):
     tiles_per = ta * tb
     # the SIMT kernel runs eight warp tiles side by side in a CTA; its leading
     # dimensions are odd, as three in four arbitrary sizes are not multiples of 4
-    simt_warp = mode == "simt" and cfg < 7
+    simt_warp = mode == "simt" and cfg < 2
     n = max(1, -(-waves * slots * (8 if simt_warp else 1) // tiles_per))
     ra, rb = bm * ta, bn * tb
     M, N = (rb, ra) if swap else (ra, rb)

@@ -72,10 +72,8 @@ cudaError_t pdl_launch(void (*kernel)(Params...), int grid, int threads, size_t 
 #endif
 
 // ---------------------------------------------------------------- SIMT ----
-// Tile configurations of the FP32 SIMT kernel.  The 128 x 128 tile (id 7) and
-// the thin ones (ids 8 and 9, for M <= 8 and N <= 8) are computed by a CTA of
-// 256 threads, the others by one warp (eight run side by side in a CTA): ids 1
-// to 6 as 32 x 32 parts in turn.
+// Tile configurations of the FP32 SIMT kernel.  Ids 0 and 1 are computed by one
+// warp (eight run side by side in a CTA), the others by a CTA of 256 threads.
 struct SimtCfg {
   int bm, bn;  // tile
   int lm, ln;  // log2 of these
@@ -88,19 +86,17 @@ constexpr SimtCfg kSimtCfgs[kSimtNumCfgs] = {
     {64, 128, 6, 7, 16, 16}, {128, 128, 7, 7, 32, 16}, {8, 128, 3, 7, 8, 16},
     {128, 8, 7, 3, 16, 8},
 };
-__host__ __device__ constexpr bool simt_warp_cfg(int cfg) { return cfg < 7; }
-// What the planners choose from: ids 2 to 6 run only when forced (their parts
-// in turn are no faster than tiles of their own); a thin matrix takes a thin
-// tile or, where even that is mostly padding, 16 x 16 ones (K = 4096 and M or
+__host__ __device__ constexpr bool simt_warp_cfg(int cfg) { return cfg < 2; }
+// What the planners choose from: ids 2 to 6 run only when forced (64 x 64 as a
+// choice of its own gained a third on one batch in 90, a large matrix of odd
+// leading dimensions among 49 small ones, and lost on as many as it won of the
+// others); a thin matrix takes a thin tile or, where even that is mostly padding, 16 x 16 ones (K = 4096 and M or
 // N <= 8, two batches of about 100 each: 568 and 474 us in thin tiles, 664 and
 // 610 in 16 x 16, 857 and 875 in 32 x 32).
 __host__ __device__ constexpr bool simt_auto_cfg(int cfg, int M, int N) {
   return cfg == 0 || (cfg == 8 ? M <= 8 : cfg == 9 ? N <= 8
                                                    : (cfg == 1 || cfg == 7) && M > 8 && N > 8);
 }
-// ids 1 to 6: 32-row and 32-column parts of a tile (one hex digit each)
-__host__ __device__ constexpr int simt_part_rows(int cfg) { return (0x2421210 >> (4 * cfg)) & 15; }
-__host__ __device__ constexpr int simt_part_cols(int cfg) { return (0x4222110 >> (4 * cfg)) & 15; }
 
 struct SimtParams {
   const MatDesc* descs;

@@ -2,14 +2,13 @@
 // staging, the FMA loop, the C read and write, and how a CTA's warps share
 // the tile queue.
 //
-// A tile is computed by a team: the whole CTA (256 threads) for the 128 x 128
-// tile and the thin ones, one warp for the small ones, so that a small tile
-// still gives every thread 8 to 32 outputs and eight tiles run side by side in
-// a CTA.  A warp's lanes form an LX x LY grid and each thread owns TM x TN
-// outputs.  The thin tiles (8 x 128, 128 x 8) are bound by the bytes they read
-// for a few FMAs each: all eight warps share one tile's long operand, in
-// slices of 32 k, so that a CTA keeps 55 KB on the way and a long K ends soon
-// (run_thin).
+// A tile is computed by a team: one warp for the 16 x 16 and 32 x 32 tiles, so
+// that a small tile still gives every thread 8 to 32 outputs and eight tiles
+// run side by side in a CTA, the whole CTA (256 threads) for all others.  A
+// warp's lanes form an LX x LY grid and each thread owns TM x TN outputs.  The
+// thin tiles (8 x 128, 128 x 8) are bound by the bytes they read for a few
+// FMAs each: all eight warps share one tile's long operand, in slices of 32 k,
+// so that a CTA keeps 55 KB on the way and a long K ends soon (run_thin).
 // Operands stream through a cp.async ring of BK k-slices:
 //   A slice: [k][BM]      rows contiguous, 16-byte cp.async when lda % 4 == 0
 //                         and A is 16-byte aligned, 4-byte otherwise
@@ -49,8 +48,9 @@ constexpr int kWarps = kThreads / 32;
 // 227 KB; a warp's tile uses its own 14 KB, a CTA tile all of it.
 constexpr int kWarpFloats = 3584;
 // Behind it the CTA's control words: the item of the next round, the number of
-// CTA tiles that warps left, and those tiles.
-constexpr int kCtlItem = 0, kCtlPosts = 1, kCtlPost = 2, kCtlInts = 16;
+// CTA tiles that warps left, those tiles, and which warp pulls first.
+constexpr int kCtlItem = 0, kCtlPosts = 1, kCtlPost = 2, kCtlTurn = 10, kCtlInts = 16;
+static_assert(kCtlPost + kWarps <= kCtlTurn, "control words");
 constexpr int kSmemBytes = kWarps * kWarpFloats * 4 + kCtlInts * 4;
 static_assert(kSimtRingCap >= 2 && kSimtRingCap <= 32, "SIMT ring cap out of range");
 
@@ -496,6 +496,12 @@ __device__ __forceinline__ int pull_item(const SimtParams& p) {
   return atomicAdd(p.counters, 1) + (int)gridDim.x;
 }
 constexpr int kNoItem = 0x7fffffff;
+// K above which a 16 x 16 tile takes slices of 32 k instead of 16: fewer waits
+// and address sums per k, but more copies before the first FMA.  One tile of K
+// = 4096 77 us in slices of 16, 65 in slices of 32; with the line at 32 and not
+// at 256, batches of some hundred matrices of 2 to 100 took up to 1.15 times as
+// long.
+constexpr int kShortK = 256;
 
 // One tile of matrix `mat` whose first row and column are m0 and n0, by the
 // calling team.  With `pull` the team's first thread takes its next item while
@@ -695,6 +701,23 @@ __device__ __forceinline__ int run_thin(const SimtParams& p, int mat, int m0, in
   }
 }
 
+// Tiles that run only when a plan asks for them, by the CTA as well.
+template <bool TA, bool TB>
+__device__ __noinline__ int run_forced(const SimtParams& p, TileItem ti, int cfg, bool pull) {
+  switch (cfg) {
+    case 2:
+      return run_tile<Shape<2, 4, 8, 4, 2, TA, TB>>(p, ti.mat, ti.tm * 64, ti.tn * 32, pull);
+    case 3:
+      return run_tile<Shape<2, 4, 4, 4, 2, TA, TB>>(p, ti.mat, ti.tm * 32, ti.tn * 64, pull);
+    case 4:
+      return run_tile<Shape<2, 4, 8, 4, 4, TA, TB>>(p, ti.mat, ti.tm * 64, ti.tn * 64, pull);
+    case 5:
+      return run_tile<Shape<4, 2, 4, 8, 4, TA, TB>>(p, ti.mat, ti.tm * 128, ti.tn * 64, pull);
+    default:
+      return run_tile<Shape<2, 4, 4, 8, 4, TA, TB>>(p, ti.mat, ti.tm * 64, ti.tn * 128, pull);
+  }
+}
+
 // The persistent kernel's body.  CTAs pull items of the largest-first queue
 // with an atomic counter.  A CTA tile occupies all eight warps.  When the
 // pulled item is a warp tile, the warps go on by themselves, each pulling and
@@ -705,13 +728,24 @@ template <bool TA, bool TB>
 __device__ __forceinline__ void persistent_body(const SimtParams& p) {
   pdl_wait();
   volatile int* ctl = control();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31;
   const int n_items = p.n_items_dev ? *p.n_items_dev : p.n_items;
   // With no more items than CTAs each CTA has its own: nobody pulls (a count of
   // CTA tiles that is not zero keeps the warps from it) and the queue's
   // counters are not touched.  16 matrices of at most 32: 4.7 us a launch with
   // every warp's pull and the count of the CTAs that finished, 3.5 without.
-  if (threadIdx.x == 0) ctl[kCtlPosts] = n_items > (int)gridDim.x ? 0 : -1;
+  // Else no more warps of a CTA pull at its start than items fall to it, all
+  // eight of the first CTAs would pull a short queue empty; and they take turns
+  // from the quarter of the SM on whose scheduler the SM's other CTA does not
+  // start, since two warps of 32 x 32 tiles on one take twice as long.  (512
+  // tiles of 8 matrices of 256 x 256 x 1024 on 304 CTAs: 112 us with eight
+  // pullers, 66 with two, 45 with their turns; only speed hangs on the slots.)
+  if (threadIdx.x == 0) {
+    ctl[kCtlPosts] = n_items > (int)gridDim.x ? 0 : -1;
+    int slot;  // of the SM's warps; warp w of a CTA has quarter (slot + w) % 4
+    asm volatile("mov.u32 %0, %%warpid;" : "=r"(slot));
+    ctl[kCtlTurn] = slot + (slot & 8) / 4;
+  }
   __syncthreads();
   int it = (int)blockIdx.x;
 #pragma unroll 1
@@ -719,8 +753,10 @@ __device__ __forceinline__ void persistent_body(const SimtParams& p) {
     int posts = 1;  // CTA tiles to compute: `it`, or those that warps left
     const bool left = simt_warp_cfg(p.descs[p.items[it].mat].cfg);
     if (left) {
-      if (warp != 0)
-        it = n_items > (int)gridDim.x
+      const int warp = threadIdx.x >> 5;
+      const int turn = ((warp + ctl[kCtlTurn]) & 3) | (warp & 4);
+      if (turn != 0)
+        it = n_items > turn * (int)gridDim.x || (it != (int)blockIdx.x && n_items > (int)gridDim.x)
                  ? __shfl_sync(0xffffffffu, lane == 0 ? pull_item(p) : 0, 0)
                  : kNoItem;
 #pragma unroll 1
@@ -733,25 +769,13 @@ __device__ __forceinline__ void persistent_body(const SimtParams& p) {
             ctl[kCtlPost + atomicAdd(const_cast<int*>(ctl) + kCtlPosts, 1)] = it;
           break;
         }
-        if (cfg == 0) {
+        if (cfg != 0)
+          next = run_tile<Shape<1, 1, 4, 8, 4, TA, TB>>(p, ti.mat, ti.tm * 32, ti.tn * 32, true);
+        else if (p.descs[ti.mat].K > kShortK)
+          next = run_tile<Shape<1, 1, 4, 4, 2, TA, TB, 32>>(p, ti.mat, ti.tm * 16, ti.tn * 16, true);
+        else
           next = run_tile<Shape<1, 1, 4, 4, 2, TA, TB>>(p, ti.mat, ti.tm * 16, ti.tn * 16, true);
-          // the staged C has been read: the next tile's copies may land there
-          __syncwarp();
-        } else {
-          // ids 1 to 6: 32 x 32 parts in turn (1 x 1, 2 x 1, 1 x 2, ...); the
-          // first is inside the matrix, the last may not be
-          const MatDesc d = p.descs[ti.mat];
-          const int bm = simt_part_rows(cfg), bn = simt_part_cols(cfg);
-          next = kNoItem;
-#pragma unroll 1
-          for (int q = bm * bn - 1; q >= 0; --q) {
-            const int m0 = (ti.tm * bm + q % bm) * 32, n0 = (ti.tn * bn + q / bm) * 32;
-            if (m0 < d.M && n0 < d.N) {
-              next = run_tile<Shape<1, 1, 4, 8, 4, TA, TB>>(p, ti.mat, m0, n0, q == 0);
-              __syncwarp();
-            }
-          }
-        }
+        __syncwarp();  // the staged C has been read: the next tile's copies may land there
         it = __shfl_sync(0xffffffffu, next, 0);
       }
       __syncthreads();
@@ -769,8 +793,10 @@ __device__ __forceinline__ void persistent_body(const SimtParams& p) {
         next = run_thin<TA, TB, false>(p, ti.mat, ti.tm * 8, ti.tn * 128, pull);
       else if (cfg == 9)
         next = run_thin<!TB, !TA, true>(p, ti.mat, ti.tn * 8, ti.tm * 128, pull);
-      else
+      else if (cfg == 7)
         next = run_tile<Shape<2, 4, 8, 8, 8, TA, TB>>(p, ti.mat, ti.tm * 128, ti.tn * 128, pull);
+      else
+        next = run_forced<TA, TB>(p, ti, cfg, pull);
     }
     if (threadIdx.x == 0) {
       ctl[kCtlItem] = next;

@@ -121,14 +121,18 @@ __host__ __device__ inline long long simt_tiles(int M, int N, SimtCfg g) {
 __host__ __device__ inline float simt_tile_ns(int K, TileCost t) {
   return fmaf(t.b_ns, (float)K, t.a_ns);
 }
-// The time a tile takes itself, with the SM nearly to itself, as the last ones
-// run (measured on thin matrices of K = 4096: 38, 55, 94, 33 and 30 ns per k
-// for ids 0, 1, 7, 8, 9, the 128 x 128 tile between that and its busy 219 ns;
-// on 16 matrices of at most 32: 2.4 us a tile of id 0 and 3.6 of id 1).
-__host__ __device__ inline float simt_alone_ns(int K, TileCost t, int c) {
-  const float f = c == 0 ? 4.5f : c < 7 ? 3.0f : c == 7 ? 0.6f : 0.75f;
-  return fmaf(t.b_ns * f, (float)K, t.a_ns * (c == 0 ? 3.0f : c < 7 ? 4.5f : f));
-}
+// What the longest tile adds to the makespan: about the time that it takes
+// beside few others, as those of a short queue and the last ones of a long one
+// do.  (With an SM to itself, K of 64 to 4096, the mean over aligned and odd
+// leading dimensions and every storage: 16.0, 35.3, 97, 22.5 and 20.5 ns per k
+// for ids 0, 1, 7, 8, 9.  Over 125 batches of 1 to 2000 matrices of sizes up to
+// 2000, against one build's times: 0.922 in the geometric mean with 25, 45 and
+// 120 for the first three and nowhere over 1.06; 0.927 with 36, 51 and 126;
+// 0.918 with 16, 40 and 107, but 1.21 on a batch of small matrices.  Ids 2 to
+// 6, which are only forced, have theirs alone.)
+constexpr TileCost kSimtTailNs[kSimtNumCfgs] = {
+    {1500.0f, 25.0f}, {2400.0f, 45.0f}, {2100.0f, 30.0f}, {2100.0f, 30.0f}, {2700.0f, 45.0f},
+    {3400.0f, 70.0f}, {3400.0f, 70.0f}, {3664.0f, 120.0f}, {2400.0f, 22.5f}, {2100.0f, 20.5f}};
 // All tiles of a matrix.  A ragged edge's FMAs are skipped in steps of gm x gn
 // outputs, its copies are not.
 __host__ __device__ inline float simt_work_ns(int M, int N, int K, SimtCfg g, TileCost t) {
@@ -149,7 +153,7 @@ __host__ __device__ inline void simt_cand(int M, int N, int K, int force, SimtCa
   e->lat[C] = -1.0f;
   if ((force >= 0 ? C != force : !simt_auto_cfg(C, M, N)) || !simt_fits(M, N, g)) return;
   e->work[C] = simt_work_ns(M, N, K, g, t);
-  e->lat[C] = simt_alone_ns(K, t, C);
+  e->lat[C] = simt_tile_ns(K, kSimtTailNs[C]);
 }
 template <int... C>
 __host__ __device__ inline void simt_cands_of(std::integer_sequence<int, C...>, int M, int N,
