@@ -65,6 +65,10 @@ struct FwTcScratch {
 
 __host__ __device__ __forceinline__ int cdiv(int a, int b) { return (a + b - 1) / b; }
 
+__host__ __device__ __forceinline__ int fwtc_strips(int M, int N) {
+  return cdiv(M, 32) + cdiv(N, 32);
+}
+
 // What the planner decides for one matrix, independently of the others; the
 // kernel then reserves queue slots, strips and workspace with atomics, and a
 // host replay (bgemm_debug_framework_tc_plan) with plain sums.
@@ -116,9 +120,49 @@ __host__ __device__ inline FwTcMat fwtc_plan_matrix(int M, int N, int K, int max
     r.a_bytes = ((unsigned long long)M * r.kpad * esz + 255) & ~255ull;
     r.b_bytes = ((unsigned long long)N * r.kpad * esz + 255) & ~255ull;
     r.kbin = min(kBins - 1, quarter_octave((float)K));
-    r.strips = cdiv(M, 32) + cdiv(N, 32);
+    r.strips = fwtc_strips(M, N);
   }
   return r;
+}
+
+// What the bins hold beside the strips, for the division of the packing (the
+// rule is in tc_common.h, along whole bins of K from the longest down): tiles,
+// raw KB and tile time (64 ns units; 32-bit, as 64-bit shared atomics are
+// compare-and-swap loops: with them the kernel took 66 us for 1000 matrices).
+struct FwTcBins {
+  int jobs[kBins], tiles[kBins], kb[kBins], time[kBins];
+};
+__host__ __device__ inline int fwtc_raw_kb(const FwTcMat& r) {
+  return (int)((4ll * ((long long)r.desc.M + r.desc.N) * r.desc.K + 1023) >> 10);
+}
+__host__ __device__ inline int fwtc_time(const FwTcMat& r, const TileCost* cost) {
+  const TileCost c = cost[r.desc.cfg];
+  return (int)((float)r.tiles * fmaf(c.b_ns, (float)r.desc.K, c.a_ns) * (1.0f / 64.0f));
+}
+// Down to and with bin `me`: strips, tiles and packing time; `late`: how far
+// that packing ends behind the GEMM's arrival at the bin, if all were fused.
+struct FwTcPrefix {
+  int jobs = 0, tiles = 0;
+  float pack = 0.0f, late = 0.0f;
+};
+__host__ __device__ inline FwTcPrefix fwtc_prefix(const FwTcBins& h, int me, int clusters) {
+  FwTcPrefix r;
+  float gemm = 0.0f;
+#pragma unroll 8
+  for (int b = kBins - 1; b >= 0; --b) {
+    if (b >= me) {
+      r.pack = fmaf((float)h.kb[b], (float)(1024.0 / kFuseBytesPerNs), r.pack);
+      r.tiles += h.tiles[b];
+      r.jobs += h.jobs[b];
+    }
+    if (b > me) gemm = fmaf((float)h.time[b], 64.0f / (float)clusters, gemm);
+  }
+  r.late = r.pack - gemm;
+  return r;
+}
+// Whether the pre-pass kernel packs no further than the prefix's bin.
+__host__ __device__ inline bool fwtc_head_ends(const FwTcPrefix& r, float late, int clusters) {
+  return r.tiles >= kHeadTiles * clusters && r.pack >= late;
 }
 
 __global__ void fwtc_plan_kernel(const int* __restrict__ dM, const int* __restrict__ dN,
@@ -126,19 +170,15 @@ __global__ void fwtc_plan_kernel(const int* __restrict__ dM, const int* __restri
                                  int mode, int clusters, FwTcScratch s) {
   __shared__ int bin_tiles[kBins];
   __shared__ int bin_start[kBins];
-  __shared__ int kbin_jobs[kBins];  // pre-pass strips per quarter-octave of K
+  __shared__ FwTcBins kbin;  // by quarter-octave of K
   __shared__ int kbin_start[kBins];
-  // for the division of the packing: the bins' tiles, raw KB and tile time (64
-  // ns units; 32-bit, as 64-bit shared atomics are compare-and-swap loops: with
-  // them the kernel took 66 us for 1000 matrices)
-  __shared__ int kbin_tiles[kBins], kbin_kb[kBins], kbin_time[kBins];
   __shared__ unsigned long long ws_total;
   __shared__ int head_bin;  // bins below it are the GEMM kernel's to pack
   __shared__ float late_w[kBins / 32];
   pdl_trigger();
   if (threadIdx.x < kBins)
-    bin_tiles[threadIdx.x] = kbin_jobs[threadIdx.x] = kbin_tiles[threadIdx.x] =
-        kbin_kb[threadIdx.x] = kbin_time[threadIdx.x] = 0;
+    bin_tiles[threadIdx.x] = kbin.jobs[threadIdx.x] = kbin.tiles[threadIdx.x] =
+        kbin.kb[threadIdx.x] = kbin.time[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
     ws_total = 0;
     head_bin = 0;
@@ -177,13 +217,10 @@ __global__ void fwtc_plan_kernel(const int* __restrict__ dM, const int* __restri
       pd.a_lo = parts == 2 ? (long long)(off + r.a_bytes) : pd.a_hi;
       pd.b_hi = (long long)(off + parts * r.a_bytes);
       pd.b_lo = parts == 2 ? (long long)(off + parts * r.a_bytes + r.b_bytes) : pd.b_hi;
-      js = atomicAdd(&kbin_jobs[r.kbin], r.strips);
-      const TileCost c = c_tc_cost[mode - 1][r.desc.cfg];
-      atomicAdd(&kbin_tiles[r.kbin], r.tiles);
-      atomicAdd(&kbin_kb[r.kbin],
-                (int)((4ll * ((long long)r.desc.M + r.desc.N) * r.desc.K + 1023) >> 10));
-      atomicAdd(&kbin_time[r.kbin],
-                (int)((float)r.tiles * fmaf(c.b_ns, (float)r.desc.K, c.a_ns) * (1.0f / 64.0f)));
+      js = atomicAdd(&kbin.jobs[r.kbin], r.strips);
+      atomicAdd(&kbin.tiles[r.kbin], r.tiles);
+      atomicAdd(&kbin.kb[r.kbin], fwtc_raw_kb(r));
+      atomicAdd(&kbin.time[r.kbin], fwtc_time(r, c_tc_cost[mode - 1]));
     }
     s.pdescs[i] = pd;
     s.job_start[i] = js;
@@ -192,41 +229,32 @@ __global__ void fwtc_plan_kernel(const int* __restrict__ dM, const int* __restri
   __syncthreads();
   // per bin: queue slots of longer tiles, strips of longer K, and the packing
   // and GEMM time up to it
-  float pack = 0.f, gemm = 0.f, late = 0.f;
-  int tiles = 0, jobs = 0;
+  FwTcPrefix pre;
   if (threadIdx.x < kBins) {
     const int me = threadIdx.x;
     int run = 0;
 #pragma unroll 8
-    for (int b = kBins - 1; b >= 0; --b) {
-      run += b > me ? bin_tiles[b] : 0;
-      if (b >= me) {
-        pack += (float)kbin_kb[b] * (float)(1024.0 / kFuseBytesPerNs);
-        tiles += kbin_tiles[b];
-        jobs += kbin_jobs[b];
-      }
-      if (b > me) gemm += (float)kbin_time[b] * (64.0f / (float)clusters);
-    }
+    for (int b = kBins - 1; b >= 0; --b) run += b > me ? bin_tiles[b] : 0;
     bin_start[me] = run;
-    kbin_start[me] = jobs - kbin_jobs[me];
-    late = pack - gemm;
+    pre = fwtc_prefix(kbin, me, clusters);
+    kbin_start[me] = pre.jobs - kbin.jobs[me];
+    float late = pre.late;
     for (int o = 16; o; o >>= 1) late = fmaxf(late, __shfl_xor_sync(0xffffffffu, late, o));
     if (lane == 0) late_w[me >> 5] = late;
     if (me == 0) {
       const bool fits = ws_total <= s.cap_ws;
       if (!fits) atomicOr(s.err, 2);
       s.counts[0] = fits ? run + bin_tiles[0] : 0;
-      s.counts[1] = fits ? jobs : 0;
-      s.counts[2] = fits ? jobs : 0;
+      s.counts[1] = fits ? pre.jobs : 0;
+      s.counts[2] = fits ? pre.jobs : 0;
     }
   }
   __syncthreads();
-  if (threadIdx.x < kBins) {
-    late = fmaxf(0.f, fmaxf(late_w[0], late_w[1]));
-    if (tiles >= kHeadTiles * clusters && pack >= late) atomicMax(&head_bin, (int)threadIdx.x);
-  }
+  if (threadIdx.x < kBins &&
+      fwtc_head_ends(pre, fmaxf(0.0f, fmaxf(late_w[0], late_w[1])), clusters))
+    atomicMax(&head_bin, (int)threadIdx.x);
   __syncthreads();
-  if (threadIdx.x == head_bin && s.counts[1] > 0) s.counts[2] = jobs;
+  if (threadIdx.x == head_bin && s.counts[1] > 0) s.counts[2] = pre.jobs;
   for (int i = threadIdx.x; i < batch; i += blockDim.x) {
     const int off = s.mat_start[i];
     if (off >= 0) s.mat_start[i] = bin_start[s.bins[i] & 0xff] + off;
@@ -234,7 +262,7 @@ __global__ void fwtc_plan_kernel(const int* __restrict__ dM, const int* __restri
     if (js >= 0) {
       const int kb = s.bins[i] >> 8;
       s.job_start[i] = kbin_start[kb] + js;
-      if (kb < head_bin) s.pdescs[i].await = cdiv(s.descs[i].M, 32) + cdiv(s.descs[i].N, 32);
+      if (kb < head_bin) s.pdescs[i].await = fwtc_strips(s.descs[i].M, s.descs[i].N);
     }
   }
 }
@@ -571,6 +599,44 @@ extern "C" int bgemm_debug_framework_tc_plan(const int* M, const int* N, const i
     }
   }
   return n_items;
+}
+
+// Host replay of fwtc_plan_kernel's division of the packing.
+extern "C" int bgemm_debug_framework_tc_division(const int* M, const int* N, const int* K,
+                                                 int batch, int max_dim, int max_k,
+                                                 long long max_operand_elems, int mode,
+                                                 int clusters, int* n_jobs, int* head_jobs,
+                                                 int* await_out) {
+  if (batch < 0 || mode < BGEMM_MODE_TF32 || mode > BGEMM_MODE_BF16X3 || clusters < 1 ||
+      !n_jobs || !head_jobs || (batch > 0 && (!M || !N || !K || !await_out)))
+    return -1;
+  TileCost cost[3][16];
+  fwtc_cost_table(cost);
+  size_t cap_items, cap_jobs, cap_ws;
+  fwtc_capacity(batch, max_dim, max_k, max_operand_elems, mode, &cap_items, &cap_jobs, &cap_ws);
+  std::vector<FwTcMat> r(batch);
+  FwTcBins h{};
+  unsigned long long ws = 0;
+  for (int i = 0; i < batch; ++i) {
+    r[i] = fwtc_plan_matrix(M[i], N[i], K[i], max_dim, max_k, mode, cost[mode - 1]);
+    if (!r[i].strips) continue;
+    ws += (mode == BGEMM_MODE_TF32 ? 1 : 2) * (r[i].a_bytes + r[i].b_bytes);
+    h.jobs[r[i].kbin] += r[i].strips;
+    h.tiles[r[i].kbin] += r[i].tiles;
+    h.kb[r[i].kbin] += fwtc_raw_kb(r[i]);
+    h.time[r[i].kbin] += fwtc_time(r[i], cost[mode - 1]);
+  }
+  float late = 0.0f;
+  for (int b = 0; b < kBins; ++b) late = std::max(late, fwtc_prefix(h, b, clusters).late);
+  int head_bin = 0;
+  for (int b = 0; b < kBins; ++b)
+    if (fwtc_head_ends(fwtc_prefix(h, b, clusters), late, clusters)) head_bin = b;
+  const bool fits = ws <= cap_ws;
+  *n_jobs = fits ? fwtc_prefix(h, 0, clusters).jobs : 0;
+  *head_jobs = fits ? fwtc_prefix(h, head_bin, clusters).jobs : 0;
+  for (int i = 0; i < batch; ++i)
+    await_out[i] = r[i].strips && r[i].kbin < head_bin ? fwtc_strips(M[i], N[i]) : 0;
+  return 0;
 }
 
 // The compile-time schedule parameters of tile_table.h as built.

@@ -323,13 +323,11 @@ static bgemm_status_t plan_batch(bgemm_plan_s* p, const int* M, const int* N, co
 static bgemm_plan_options_t default_options();
 
 // Host-only replay of the tensor-core planner with a given number of one-SM
-// slots and CTA pairs (tests; no GPU needed).  Returns the number of items,
-// or -1 on error / overflow.
-int debug_tc_plan(const int* M, const int* N, const int* K, int batch, int mode, int family,
-                  int slots, int clusters, int* cfg_out, int* items_out, int max_items,
-                  long long* ws_out, int* jobs_out, int max_jobs, int* n_jobs,
-                  long long* ws_bytes, int* pair) {
-  if (mode < BGEMM_MODE_TF32 || mode > BGEMM_MODE_BF16X3 || slots < 1 || clusters < 0) return -1;
+// slots and CTA pairs (tests; no GPU needed), handed to `read` when it went
+// well; p's tensor-core plan is released afterwards.
+template <typename Read>
+static bgemm_status_t replay_tc_plan(const int* M, const int* N, const int* K, int batch, int mode,
+                                     int family, int slots, int clusters, const Read& read) {
   std::vector<int> ld(batch);
   for (int i = 0; i < batch; ++i) ld[i] = std::max(1, std::max(M[i], K[i]));
   bgemm_plan_s p;
@@ -341,8 +339,20 @@ int debug_tc_plan(const int* M, const int* N, const int* K, int batch, int mode,
   bgemm_status_t st = tc_init(&p, &p.opt, clusters);
   if (st == BGEMM_SUCCESS)
     st = plan_batch(&p, M, N, K, ld.data(), ld.data(), ld.data(), batch, true, bp);
+  if (st == BGEMM_SUCCESS) read(p, bp);
+  if (p.tc) tc_plan_release(&p);
+  return st;
+}
+
+// Returns the number of items, or -1 on error / overflow.
+int debug_tc_plan(const int* M, const int* N, const int* K, int batch, int mode, int family,
+                  int slots, int clusters, int* cfg_out, int* items_out, int max_items,
+                  long long* ws_out, int* jobs_out, int max_jobs, int* n_jobs,
+                  long long* ws_bytes, int* pair) {
+  if (mode < BGEMM_MODE_TF32 || mode > BGEMM_MODE_BF16X3 || slots < 1 || clusters < 0) return -1;
   int n = -1;
-  if (st == BGEMM_SUCCESS) {
+  replay_tc_plan(M, N, K, batch, mode, family, slots, clusters,
+                 [&](bgemm_plan_s& p, const BatchPlan& bp) {
     n = bp.req.tiles;
     for (int i = 0; cfg_out && i < batch; ++i)
       cfg_out[i] = (M[i] && N[i]) ? bp.descs[i].cfg | (bp.descs[i].aux & kTcSwapFlag ? 1 << 8 : 0)
@@ -360,8 +370,7 @@ int debug_tc_plan(const int* M, const int* N, const int* K, int batch, int mode,
     }
     tc_debug_layout(&p, ws_out, jobs_out, max_jobs, n_jobs, pair);
     *ws_bytes = (long long)bp.req.workspace_bytes;
-  }
-  if (p.tc) tc_plan_release(&p);
+  });
   return n;
 }
 
@@ -1296,6 +1305,33 @@ int bgemm_debug_tc_plan(const int* M, const int* N, const int* K, int batch, int
     if (M[i] < 0 || N[i] < 0 || K[i] < 0) return -1;
   return debug_tc_plan(M, N, K, batch, mode, family, slots, clusters, cfg_out, items_out,
                        max_items, ws_out, jobs_out, max_jobs, n_jobs, ws_bytes, kernel_family);
+}
+
+int bgemm_debug_tc_division(const int* M, const int* N, const int* K, int batch, int mode,
+                            int family, int slots, int clusters, int* n_jobs, int* head_jobs,
+                            int* await_out) {
+  clear_error();
+  if (batch < 0 || (batch > 0 && (!M || !N || !K || !await_out)) || !n_jobs || !head_jobs ||
+      mode < BGEMM_MODE_TF32 || mode > BGEMM_MODE_BF16X3 || slots < 1 || clusters < 0)
+    return -1;
+  for (int i = 0; i < batch; ++i)
+    if (M[i] < 0 || N[i] < 0 || K[i] < 0) return -1;
+  return replay_tc_plan(M, N, K, batch, mode, family, slots, clusters,
+                        [&](bgemm_plan_s& p, const BatchPlan&) {
+                          tc_debug_division(&p, n_jobs, head_jobs, await_out);
+                        }) == BGEMM_SUCCESS
+             ? 0
+             : -1;
+}
+
+int bgemm_debug_plan_packing(void* plan, int who) {
+  clear_error();
+  bgemm_plan_s* p = static_cast<bgemm_plan_s*>(plan);
+  if (p && p->mix_tc) p = p->mix_tc;
+  if (!p || !p->tc || who < BGEMM_DEBUG_PACKING_RULE || who > BGEMM_DEBUG_PACKING_INSIDE)
+    return -1;
+  tc_debug_packing(p, who);
+  return 0;
 }
 
 int bgemm_debug_simt_queue(const int* M, const int* N, const int* K, int batch, int slots,

@@ -113,6 +113,10 @@ bgemm_status_t choose_tiles(int ncfg, TileEval eval, const int* M, const int* N,
 bgemm_status_t tc_init(bgemm_plan_s* p, const bgemm_plan_options_t* opt, int clusters = -1);
 void tc_debug_layout(bgemm_plan_s* p, long long* ws_out, int* jobs_out, int max_jobs,
                      int* n_jobs, int* pair);
+// tc_debug_division: the pre-pass's jobs and each matrix's strips packed by the
+// GEMM kernel; tc_debug_packing: who packs from the next layout on.
+void tc_debug_division(const bgemm_plan_s* p, int* n_jobs, int* head_jobs, int* await_out);
+void tc_debug_packing(bgemm_plan_s* p, int who);
 // tc_choose: tile configurations of a batch; the first call of a plan also
 // fixes its kernel family (one-SM or CTA pair), later calls keep it.
 bgemm_status_t tc_choose(bgemm_plan_s* p, const int* M, const int* N, const int* K, int batch,

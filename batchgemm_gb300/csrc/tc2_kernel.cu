@@ -793,6 +793,16 @@ __global__ void __launch_bounds__(kThreads2, 1) tc2_gemm_kernel(const TcGemmPara
   if (p.cta_times && threadIdx.x == 0) p.cta_times[2 * blockIdx.x + 1] = gtimer();
 }
 
+// As bounded_wait_selftest_kernel (tc_kernel.cu), of wait_packed.
+__global__ void packed_wait_selftest_kernel(int* err, int* out, unsigned long long limit_ns) {
+  __shared__ int abort_flag;
+  if (threadIdx.x == 0) {
+    abort_flag = 0;
+    out[1] = wait_packed(out + 2, 1, err, &abort_flag, limit_ns) ? 1 : 0;
+    out[0] = 1;
+  }
+}
+
 template <int KIND, int SPLIT, bool BETA>
 cudaError_t launch2(const TcGemmParams& p, int grid, cudaStream_t s) {
   static bool attr = false;
@@ -835,6 +845,12 @@ cudaError_t tc2_gemm_launch(int kind, int split, const TcGemmParams& p, int grid
   if (kind == kKindTF32) return launch2b<kKindTF32, 1>(p, grid, s);
   if (kind == kKindBF16 && split) return launch2b<kKindBF16, 1>(p, grid, s);
   return cudaErrorInvalidValue;
+}
+
+cudaError_t tc2_wait_selftest_launch(int* err, int* out, unsigned long long limit_ns,
+                                     cudaStream_t s) {
+  packed_wait_selftest_kernel<<<1, 32, 0, s>>>(err, out, limit_ns);
+  return cudaGetLastError();
 }
 
 int tc2_max_clusters() {

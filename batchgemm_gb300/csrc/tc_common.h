@@ -160,5 +160,8 @@ int tc_smem_bytes(int kind, int split);
 cudaError_t tc2_gemm_launch(int kind, int split, const TcGemmParams& p, int grid,
                             cudaStream_t s);
 int tc2_max_clusters();
+// one CTA waiting for packed strips that nothing counts
+cudaError_t tc2_wait_selftest_launch(int* err, int* out, unsigned long long limit_ns,
+                                     cudaStream_t s);
 
 }  // namespace bgemm

@@ -43,6 +43,7 @@ struct TcPlan {
   std::vector<PackDesc> pd;
   std::vector<PackJob> jobs;
   int head = 0;              // jobs of the pre-pass kernel; the GEMM kernel does the rest
+  int packing = BGEMM_DEBUG_PACKING_RULE;  // who packs, from the next layout on
 };
 
 static inline long long cdiv(long long a, long long b) { return (a + b - 1) / b; }
@@ -176,7 +177,8 @@ static long long tc_tiles(const MatDesc& d, bool pair) {
 }
 // Jobs of the pre-pass kernel (the rule is in tc_common.h).
 static int tc_divide(TcPlan* t, const std::vector<MatDesc>& hd, const std::vector<int>& order) {
-  if (!t->pair) return (int)t->jobs.size();
+  if (!t->pair || t->packing == BGEMM_DEBUG_PACKING_BEFORE) return (int)t->jobs.size();
+  if (t->packing == BGEMM_DEBUG_PACKING_INSIDE) return 0;
   // packing done and GEMM begun, in ns from the GEMM kernel's start, if all
   // the packing were fused
   double pack = 0, gemm = 0, late = 0;
@@ -505,16 +507,22 @@ void tc_debug_layout(bgemm_plan_s* p, long long* ws_out, int* jobs_out, int max_
   }
   *pair = t->pair ? 2 : 1;
 }
-}  // namespace bgemm
+void tc_debug_division(const bgemm_plan_s* p, int* n_jobs, int* head_jobs, int* await_out) {
+  const TcPlan* t = p->tc;
+  *n_jobs = (int)t->jobs.size();
+  *head_jobs = t->head;
+  for (size_t i = 0; i < t->pd.size(); ++i) await_out[i] = t->pd[i].await;
+}
+void tc_debug_packing(bgemm_plan_s* p, int who) { p->tc->packing = who; }
 
-extern "C" int bgemm_debug_bounded_wait_selftest(unsigned long long limit_ns, int* error,
-                                                 int* returned, int* wait_ok) {
-  using namespace bgemm;
+// Runs a self-test kernel of a bounded wait: its error word and two results.
+static int wait_selftest(cudaError_t (*launch)(int*, int*, unsigned long long, cudaStream_t),
+                         unsigned long long limit_ns, int* error, int* returned, int* wait_ok) {
   int* d = nullptr;
   if (cudaMalloc(&d, 4 * sizeof(int)) != cudaSuccess) return -1;
   int h[4] = {0, 0, 0, 0};
   cudaError_t e = cudaMemset(d, 0, 4 * sizeof(int));
-  if (e == cudaSuccess) e = tc_wait_selftest_launch(d, d + 1, limit_ns, nullptr);
+  if (e == cudaSuccess) e = launch(d, d + 1, limit_ns, nullptr);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost);
   cudaFree(d);
@@ -523,6 +531,18 @@ extern "C" int bgemm_debug_bounded_wait_selftest(unsigned long long limit_ns, in
   if (returned) *returned = h[1];
   if (wait_ok) *wait_ok = h[2];
   return 0;
+}
+}  // namespace bgemm
+
+extern "C" int bgemm_debug_bounded_wait_selftest(unsigned long long limit_ns, int* error,
+                                                 int* returned, int* wait_ok) {
+  return bgemm::wait_selftest(bgemm::tc_wait_selftest_launch, limit_ns, error, returned, wait_ok);
+}
+
+extern "C" int bgemm_debug_packed_wait_selftest(unsigned long long limit_ns, int* error,
+                                                int* returned, int* wait_ok) {
+  return bgemm::wait_selftest(bgemm::tc2_wait_selftest_launch, limit_ns, error, returned,
+                              wait_ok);
 }
 
 extern "C" int bgemm_debug_set_tc_schedule(int mode, const int* group) {

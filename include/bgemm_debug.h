@@ -70,6 +70,32 @@ int bgemm_debug_framework_tc_plan(const int* M, const int* N, const int* K, int 
                                   long long* ws_out, int* n_jobs, long long* ws_used,
                                   long long* ws_capacity, int* err, int* cfg_out);
 
+/* How those two planners divide the operand packing of the CTA-pair kernel:
+ * of the *n_jobs strips in order, the first *head_jobs are the pre-pass
+ * kernel's, the rest are packed inside the GEMM kernel, whose tiles of matrix
+ * i wait for await_out[i] of them (0: none).  Arguments otherwise as above;
+ * with the one-SM kernel everything is the pre-pass's.  Return 0, or -1 on
+ * invalid arguments or planner errors. */
+int bgemm_debug_tc_division(const int* M, const int* N, const int* K, int batch, int mode,
+                            int family, int slots, int clusters, int* n_jobs, int* head_jobs,
+                            int* await_out);
+int bgemm_debug_framework_tc_division(const int* M, const int* N, const int* K, int batch,
+                                      int max_dim, int max_k, long long max_operand_elems,
+                                      int mode, int clusters, int* n_jobs, int* head_jobs,
+                                      int* await_out);
+
+/* Who packs a tensor-core plan's operands from its next bgemm_plan_update on:
+ * the planner's rule, all of it before the GEMM, or all of it inside the
+ * CTA-pair GEMM kernel.  For tests (the results are the same bits) and for the
+ * autotuner, which times tiles without packing.  Returns 0, or -1 for another
+ * plan or value. */
+enum {
+  BGEMM_DEBUG_PACKING_RULE = 0,
+  BGEMM_DEBUG_PACKING_BEFORE = 1,
+  BGEMM_DEBUG_PACKING_INSIDE = 2
+};
+int bgemm_debug_plan_packing(void* plan, int who);
+
 /* Cost-model entry of configuration `cfg` of `mode` (0 SIMT, 1 TF32,
  * 2 TF32X3, 3 BF16X3): modelled time of one tile = *a_ns + *b_ns * K
  * nanoseconds, as the device planners read it.  Returns 0, or -1 for an
@@ -111,6 +137,10 @@ int bgemm_debug_compare_tensor_maps(void* plan, void* stream, int* n_maps, int* 
  * if a CUDA call failed. */
 int bgemm_debug_bounded_wait_selftest(unsigned long long limit_ns, int* error, int* returned,
                                       int* wait_ok);
+
+/* The same of the wait for packed operands: a count that nothing raises. */
+int bgemm_debug_packed_wait_selftest(unsigned long long limit_ns, int* error, int* returned,
+                                     int* wait_ok);
 
 /* Promotion schedule of the split tensor-core modes on CTA pairs (mode 2
  * TF32X3, 3 BF16X3; 1 is accepted and unused): group[b] for the 8 buckets
