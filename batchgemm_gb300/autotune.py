@@ -76,7 +76,7 @@ def valid_tc(mode, cfg):
     return True
 
 
-def measure(mode, cfg, K, slots, waves=6, reps=5, hbm_gbs=6000.0):
+def measure(mode, cfg, K, slots, waves=6, reps=5):
     import torch
     from batchgemm_gb300.batch import DeviceBatch
     if mode == "simt":
@@ -100,29 +100,46 @@ def measure(mode, cfg, K, slots, waves=6, reps=5, hbm_gbs=6000.0):
     with db.plan(mode, force_tile_config=cfg, rebalance=False) as p:
         info = p.info()
         assert info["num_tiles"] == n * tiles_per, (info["num_tiles"], n * tiles_per)
-        for _ in range(2):
-            db.execute(p, 1.0, 0.0)
-        torch.cuda.synchronize()
-        e0 = torch.cuda.Event(enable_timing=True)
-        e1 = torch.cuda.Event(enable_timing=True)
+        ms = kernel_ms(db, p, mode, reps)
+        grid = info["grid"]
+    lanes = grid // 2 if (mode != "simt" and cfg >= 8) else grid
+    per_tile = ms * 1e6 * lanes / (n * tiles_per)
+    del db
+    return per_tile, ms
+
+
+def kernel_ms(db, p, mode, reps):
+    """Time (ms) of the plan's SIMT kernel (mean of `reps` executes) or GEMM kernel (the best),
+    all operands packed before the GEMM starts: inside it the packing would be timed with the
+    tiles."""
+    import torch
+    import batchgemm_gb300 as bg
+    if mode != "simt":
+        assert bg.lib().bgemm_debug_plan_packing(p._h, 1) == 0  # BGEMM_DEBUG_PACKING_BEFORE
+        p.update(db.M, db.N, db.K, db.lda, db.ldb, db.ldc)
+    for _ in range(2):
+        db.execute(p, 1.0, 0.0)
+    torch.cuda.synchronize()
+    if mode == "simt":  # executes back to back: a last wave is part of a tile's time here
+        e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
         e0.record()
         for _ in range(reps):
             db.execute(p, 1.0, 0.0)
         e1.record()
         torch.cuda.synchronize()
-        p.check_device()
-        ms = e0.elapsed_time(e1) / reps
-        grid = info["grid"]
-    t_gemm_ns = ms * 1e6
-    if mode != "simt":
-        elems = n * (M * K + N * K)
-        wbytes = {"tf32": 4, "tf32x3": 8, "bf16x3": 4}[mode]
-        t_pack_ns = elems * (4 + wbytes) / (hbm_gbs * 1e9) * 1e9
-        t_gemm_ns = max(t_gemm_ns - t_pack_ns, 0.05 * t_gemm_ns)
-    lanes = grid // 2 if (mode != "simt" and cfg >= 8) else grid
-    per_tile = t_gemm_ns * lanes / (n * tiles_per)
-    del db
-    return per_tile, ms
+        return e0.elapsed_time(e1) / reps
+    ts = []
+    for _ in range(reps):
+        e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        e0.record()
+        e1.record()
+        p.set_kernel_events(e0, e1)
+        db.execute(p, 1.0, 0.0)
+        e1.synchronize()
+        ts.append(e0.elapsed_time(e1))
+    p.set_kernel_events(None, None)
+    p.check_device()
+    return min(ts)
 
 
 def fit(Ks, ts):
@@ -138,7 +155,7 @@ SCHED_CANDIDATES = [0, 1, 2, 3, 4, 6, 8]
 
 
 def sched_measure(mode, K, group, n=24, size=1024, reps=5, samples=128):
-    """GEMM-kernel time (ms, best of reps) and sampled errors (numpy) of one
+    """GEMM-kernel time (ms) and sampled errors (numpy) of one
     promotion group length on n matrices of size x size x K."""
     import ctypes
     import torch
@@ -154,22 +171,8 @@ def sched_measure(mode, K, group, n=24, size=1024, reps=5, samples=128):
     assert L.bgemm_debug_set_tc_schedule(mid, (ctypes.c_int * 8)(*g)) == 0
     try:
         db = DeviceBatch([size] * n, [size] * n, [K] * n).fill_fast("normal", 0)
-        best = float("inf")
         with db.plan(mode, kernel_family="pair") as p:
-            for _ in range(2):
-                db.execute(p, 1.0, 0.0)
-            torch.cuda.synchronize()
-            for _ in range(reps):
-                e0 = torch.cuda.Event(enable_timing=True)
-                e1 = torch.cuda.Event(enable_timing=True)
-                e0.record()
-                e1.record()
-                p.set_kernel_events(e0, e1)
-                db.execute(p, 1.0, 0.0)
-                e1.synchronize()
-                best = min(best, e0.elapsed_time(e1))
-            p.set_kernel_events(None, None)
-            p.check_device()
+            ms = kernel_ms(db, p, mode, reps)
         err, _ = fp64_sampled_error(db, per_matrix=samples, seed=7, samples=True)
         db.C.zero_()
         with db.plan("simt") as ps:
@@ -178,7 +181,7 @@ def sched_measure(mode, K, group, n=24, size=1024, reps=5, samples=128):
         serr, _ = fp64_sampled_error(db, per_matrix=samples, seed=7, samples=True)
         del db
         torch.cuda.empty_cache()
-        return best, err, serr
+        return ms, err, serr
     finally:
         L.bgemm_debug_set_tc_schedule(mid, (ctypes.c_int * 8)(*list(prev)))
 
@@ -383,11 +386,6 @@ def main():
             write_table(args.out, simt_cur, tc_cur, sched, torch.cuda.get_device_name(0),
                         dev["num_sms"], params_cur)
         return
-    peaks = {}
-    pk = os.path.join(os.path.dirname(PKG), "MEASURED_PEAKS.json")
-    if os.path.exists(pk):
-        peaks = json.load(open(pk))
-    hbm = float(peaks.get("hbm_gbs", 6000.0))
     simt_slots = dev["num_sms"] * dev["simt_ctas_per_sm"]
     tc_slots = dev["num_sms"] * dev["tc_ctas_per_sm"]
     raw = {}
@@ -401,7 +399,7 @@ def main():
             slots = simt_slots if mode == "simt" else (tc_slots // 2 if c >= 8 else tc_slots)
             ts = []
             for K in Ks:
-                t, ms = measure(mode, c, K, slots, hbm_gbs=hbm)
+                t, ms = measure(mode, c, K, slots)
                 ts.append(t)
                 raw.setdefault(mode, {}).setdefault(str(c), []).append([K, t, ms])
             a, b = fit(Ks, ts)
