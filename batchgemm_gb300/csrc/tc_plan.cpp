@@ -37,7 +37,6 @@ struct TcPlan {
   PackJob* d_jobs = nullptr;
   int* d_err = nullptr;
   int* d_ready = nullptr;    // finished strips per matrix (reset by the GEMM kernel)
-  int n_jobs = 0;
   int pack_grid = 1;
   // layout of the last planned batch, uploaded by tc_commit
   std::vector<PackDesc> pd;
@@ -387,7 +386,6 @@ bgemm_status_t tc_commit(bgemm_plan_s* p, int stage, int batch, bool first, cuda
   if (e == cudaSuccess) e = copy(t->off_pd, sizeof(PackDesc) * (size_t)batch);
   if (e == cudaSuccess) e = copy(t->off_jobs, sizeof(PackJob) * t->jobs.size());
   if (e != cudaSuccess) return cuda_error(e, "tensor-core descriptor upload");
-  t->n_jobs = (int)t->jobs.size();
   if (!t->host_tmaps && batch > 0) {
     // per-matrix tensor maps built on the device, once per batch
     TcTmapParams tp{p->d_descs, t->d_pdescs, t->d_templ, t->d_tmaps, ws, batch, t->kind,
