@@ -347,8 +347,9 @@ __device__ __forceinline__ bool wait_packed(const int* ready, int need, int* err
   return true;
 }
 
-// BETA: the launch's beta is nonzero (C is read: late L2 prefetch, 16 reads in
-// flight).  The beta = 0 form is a separate instantiation that keeps the
+// BETA: the launch's beta is nonzero (C is read, eight reads ahead of the
+// stores; the L2 prefetch of kCPrefetchLead is off in the tuned table).  The
+// beta = 0 form is a separate instantiation that keeps the
 // plain epilogue's code (the read path's registers slowed it by ~4 %).
 template <int KIND, int SPLIT, bool BETA>
 __global__ void __launch_bounds__(kThreads2, 1) tc2_gemm_kernel(const TcGemmParams p) {

@@ -3,7 +3,8 @@
 //
 // Kernels:
 //   tc_pack_kernel  (before the GEMM below, whole; before the CTA-pair GEMM,
-//                   tc2_kernel.cu, the operands of the first tiles) splits every operand element x into hi = round(x) and
+//                   tc2_kernel.cu, the operands of the first tiles) splits
+//                   every operand element x into hi = round(x) and
 //                   lo = round(x - hi) (TF32 or BF16, round to nearest even)
 //                   and writes them K-major ("rows of K", 16-byte aligned row
 //                   length) into the plan's workspace: A is transposed from
@@ -198,13 +199,12 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(const TcPackParams p) {
       const int wk = (tid & 7) * 4;
       if (n >= rows) continue;
       const float* col = X + n * ldx;
-      const bool vec = ((reinterpret_cast<uintptr_t>(col) & 15u) == 0);
       for (int k0 = 0; k0 < K; k0 += kPackK) {
         float x[kPackK / 32][4];
 #pragma unroll
         for (int h2 = 0; h2 < kPackK / 32; ++h2) {
           const int k = k0 + wk + 32 * h2;
-          if (vec && k + 4 <= K) {
+          if (k + 4 <= K) {
             const float4 f = *reinterpret_cast<const float4*>(col + k);
             x[h2][0] = f.x; x[h2][1] = f.y; x[h2][2] = f.z; x[h2][3] = f.w;
           } else {
