@@ -31,6 +31,9 @@
  * split).  They are checked against an FP64 oracle with a sqrt(K)-scaled
  * relative tolerance.
  *
+ * C_i must not overlap any A_j or B_j of the batch, nor any other C_j, as in
+ * BLAS: a call reads operands of one tile while it stores another.
+ *
  * Ownership: the caller owns every A/B/C buffer and the device arrays of
  * device pointers dA/dB/dC; the library owns its plans, their device
  * descriptors and workspace.  All device work is asynchronous on `stream`.
