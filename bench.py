@@ -166,6 +166,22 @@ def ncu_traffic(mode, workload):
     return None
 
 
+def packing_waits(w, mode, num_sms):
+    """Per matrix: the strips of its operands that the GEMM kernel packs itself (0:
+    the pre-pass kernel packs them), as the planner divides them on this device."""
+    import ctypes
+    import batchgemm_gb300 as bg
+    n = w.batch
+    jobs, head, wait = ctypes.c_int(), ctypes.c_int(), (ctypes.c_int * n)()
+    rc = bg.lib().bgemm_debug_tc_division(
+        bg.int_array(w.M), bg.int_array(w.N), bg.int_array(w.K), n,
+        {"tf32": 1, "tf32x3": 2, "bf16x3": 3}[mode], 0, num_sms, num_sms // 2,
+        ctypes.byref(jobs), ctypes.byref(head), wait)
+    if rc != 0:
+        raise RuntimeError("bgemm_debug_tc_division failed")
+    return list(wait)
+
+
 # ------------------------------------------------------------ CPU oracle --
 def cpu_sample(w, budget_s=15.0, threads=None):
     """Times the CPU FP32 loop (the oracle port; the reference ships no CPU
@@ -306,24 +322,26 @@ def gpu_leg(args, rank, world, local):
     out.update(value=value, ms=ms_max, info=info, clocks=clocks, err=(err_max, err_mean, nsamp),
                launches=info["kernels_per_execute"] * args.steps)
     # the dominant (GEMM) kernel alone: events recorded by the library around
-    # its launch, on the stream it is launched on, over `steps` executes
+    # its launch, on the stream it is launched on, over `steps` executes; the
+    # pre-pass before it, from an event ahead of the execute to the first of these
     evs = []
     for _ in range(args.steps):
-        a = torch.cuda.Event(enable_timing=True)
-        b = torch.cuda.Event(enable_timing=True)
-        a.record(s)
-        b.record(s)
-        evs.append((a, b))
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(3)]
+        for e in ev:
+            e.record(s)
+        evs.append(ev)
     s.synchronize()
     with torch.cuda.stream(s):
-        for a, b in evs:
+        for pre, a, b in evs:
             if flush is not None:
                 flush.zero_()
+            pre.record(s)
             plan.set_kernel_events(a, b)
             db.execute(plan, w.alpha, w.beta, stream=s)
     s.synchronize()
     plan.set_kernel_events(None, None)
-    out["kernel_ms"] = sum(a.elapsed_time(b) for a, b in evs) / len(evs)
+    out["kernel_ms"] = sum(a.elapsed_time(b) for _, a, b in evs) / len(evs)
+    out["pre_pass_ms"] = sum(pre.elapsed_time(a) for pre, a, _ in evs) / len(evs)
     if args.mode != "simt":
         # load balance of the GEMM's static tile schedule: every persistent
         # CTA stamps the global timer when it starts and when it finishes
@@ -440,7 +458,7 @@ def gpu_leg(args, rank, world, local):
                    "before the timed region (batchgemm_gb300.peaks.tf32_burst)")
         ach = mult * flops / (kms * 1e-3) / 1e12
         step_ms = out["ms"]
-        pre_ms = step_ms - kms
+        pre_ms = out["pre_pass_ms"]
         pre_traffic = ncu_traffic(mode + "_pre_pass", w.name)
         out["roofline"] = {"bound": "tensor", "achieved": round(ach, 2),
                            "peak": round(pipe_peak, 1), "unit": "TFLOP/s",
@@ -457,15 +475,18 @@ def gpu_leg(args, rank, world, local):
                            "step_dram_bytes": (traffic + pre_traffic
                                                if traffic and pre_traffic else None),
                            "pre_pass_traffic": pre_traffic}
-        elems = float(sum(m * k + k * n for m, n, k in zip(w.M, w.N, w.K)))
-        pre_bytes = elems * (4 + {"tf32": 4, "tf32x3": 8, "bf16x3": 4}[mode])
-        # packing overlaps the GEMM, so its bytes are set against the whole step
-        pre_ach = pre_bytes / (step_ms * 1e-3) / 1e9
+        # the pre-pass kernel's own share of the packing; the rest is packed inside
+        # the GEMM kernel, and its time is part of kernel_ms
+        wait = packing_waits(w, mode, num_sms)
+        per_elem = 4 + {"tf32": 4, "tf32x3": 8, "bf16x3": 4}[mode]
+        elems = [float((m + n) * k) for m, n, k in zip(w.M, w.N, w.K)]
+        pre_bytes = per_elem * sum(e for e, late in zip(elems, wait) if not late)
+        pre_ach = pre_bytes / (pre_ms * 1e-3) / 1e9
         out["roofline"]["pre_pass"] = {
-            "bound": "overlapped with the GEMM", "achieved": round(pre_ach, 1),
-            "peak": out["pre_pass_peak"], "unit": "GB/s over the whole step",
-            "frac": round(pre_ach / out["pre_pass_peak"], 4),
+            "bound": "hbm", "achieved": round(pre_ach, 1), "peak": out["pre_pass_peak"],
+            "unit": "GB/s", "frac": round(pre_ach / out["pre_pass_peak"], 4),
             "algorithmic_bytes": pre_bytes,
+            "packed_in_gemm_bytes": per_elem * sum(elems) - pre_bytes,
             "peak_source": "measured in this run before the timed region: the library's float4 "
                            "streaming probe (bgemm_debug_hbm_probe) with the pre-pass's mix (%s), "
                            "1 GiB buffers, best of two grids" % out["pre_pass_mix"]}
