@@ -147,8 +147,10 @@ struct TcTmapParams {
 // 3xTF32 and TF32 the same to 1 %, the cases within 1 %.)
 // Measured: 2, 4 and 8 tiles per pair 6.81, 6.83 and 6.88 ms (a stream of four
 // batches) and 538, 525 and 534 us (96 matrices in 3xBF16); 800, 1200 and 2000
-// bytes per ns 1283, 1230 and 1235 us (128 matrices in TF32, whose GEMM is the
-// shortest beside its packing).
+// bytes per ns, one figure for the three kinds of split: TF32 1267, 1211 and
+// 1213 us (128 matrices of N = K = 1024, whose GEMM is the shortest beside its
+// packing) and 3.93, 3.71 and 3.78 ms (the 600 above), 3xBF16 4.20, 4.15 and
+// 4.21 ms, 3xTF32 the same to 2 %, the other cases to 0.5 %.
 constexpr int kHeadTiles = 4;
 constexpr double kFuseBytesPerNs = 1200.0;
 
