@@ -496,12 +496,6 @@ __device__ __forceinline__ int pull_item(const SimtParams& p) {
   return atomicAdd(p.counters, 1) + (int)gridDim.x;
 }
 constexpr int kNoItem = 0x7fffffff;
-// K above which a 16 x 16 tile takes slices of 32 k instead of 16: fewer waits
-// and address sums per k, but more copies before the first FMA.  One tile of K
-// = 4096 77 us in slices of 16, 65 in slices of 32; with the line at 32 and not
-// at 256, batches of some hundred matrices of 2 to 100 took up to 1.15 times as
-// long.
-constexpr int kShortK = 256;
 
 // One tile of matrix `mat` whose first row and column are m0 and n0, by the
 // calling team.  With `pull` the team's first thread takes its next item while
@@ -771,7 +765,7 @@ __device__ __forceinline__ void persistent_body(const SimtParams& p) {
         }
         if (cfg != 0)
           next = run_tile<Shape<1, 1, 4, 8, 4, TA, TB>>(p, ti.mat, ti.tm * 32, ti.tn * 32, true);
-        else if (p.descs[ti.mat].K > kShortK)
+        else if (p.descs[ti.mat].K > kSimtShortK)
           next = run_tile<Shape<1, 1, 4, 4, 2, TA, TB, 32>>(p, ti.mat, ti.tm * 16, ti.tn * 16, true);
         else
           next = run_tile<Shape<1, 1, 4, 4, 2, TA, TB>>(p, ti.mat, ti.tm * 16, ti.tn * 16, true);
