@@ -763,12 +763,14 @@ __device__ __forceinline__ void persistent_body(const SimtParams& p) {
             ctl[kCtlPost + atomicAdd(const_cast<int*>(ctl) + kCtlPosts, 1)] = it;
           break;
         }
-        if (cfg != 0)
-          next = run_tile<Shape<1, 1, 4, 8, 4, TA, TB>>(p, ti.mat, ti.tm * 32, ti.tn * 32, true);
-        else if (p.descs[ti.mat].K > kSimtShortK)
+        // (16 x 16: slices of 32 k, fewer waits and address sums per k.  One tile
+        // of K = 4096 66 us, in slices of 16 78.  Both forms, by a line at K =
+        // 256, cost batches that run only one of them up to a tenth: 546 matrices
+        // of up to 109 11.3 us, 9.9 and 10.7 with either alone.)
+        if (cfg == 0)
           next = run_tile<Shape<1, 1, 4, 4, 2, TA, TB, 32>>(p, ti.mat, ti.tm * 16, ti.tn * 16, true);
         else
-          next = run_tile<Shape<1, 1, 4, 4, 2, TA, TB>>(p, ti.mat, ti.tm * 16, ti.tn * 16, true);
+          next = run_tile<Shape<1, 1, 4, 8, 4, TA, TB>>(p, ti.mat, ti.tm * 32, ti.tn * 32, true);
         __syncwarp();  // the staged C has been read: the next tile's copies may land there
         it = __shfl_sync(0xffffffffu, next, 0);
       }

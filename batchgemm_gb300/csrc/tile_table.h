@@ -123,34 +123,20 @@ __host__ __device__ inline long long simt_tiles(int M, int N, SimtCfg g) {
 __host__ __device__ inline float simt_tile_ns(int K, TileCost t) {
   return fmaf(t.b_ns, (float)K, t.a_ns);
 }
-// K above which a 16 x 16 tile takes slices of 32 k instead of 16: fewer waits
-// and address sums per k, but more copies before the first FMA.  One tile of K
-// = 4096 77 us in slices of 16, 65 in slices of 32; with the line at 32 and not
-// at 256, batches of some hundred matrices of 2 to 100 took up to 1.15 times as
-// long.
-constexpr int kSimtShortK = 256;
 // What the longest tile adds to the makespan: about the time that it takes
 // beside few others, as those of a short queue and the last ones of a long one
 // do.  (With an SM to itself, K of 64 to 4096, the mean over aligned and odd
 // leading dimensions and every storage: 16.0, 35.3, 97, 22.5 and 20.5 ns per k
-// for ids 0, 1, 7, 8, 9.  Over 125 batches of 1 to 2000 matrices of sizes up to
-// 2000, against one build's times: 0.922 in the geometric mean with 25, 45 and
-// 120 for the first three and nowhere over 1.06; 0.927 with 36, 51 and 126;
-// 0.918 with 16, 40 and 107, but 1.21 on a batch of small matrices.  Ids 2 to
-// 6, which are only forced, have theirs alone.)
+// for ids 0, 1, 7, 8, 9.  125 batches of 1 to 2000 matrices of sizes up to
+// 2000, against one build's times, with 25, 45 and 120 for the first three
+// 0.922 in the geometric mean, with 36, 51 and 126 0.927.  Id 0 has its own 16
+// since it takes slices of 32 k at any K: 149 batches of up to 4 GFLOP 0.975
+// against 25; a first part of 1500 ns instead 0.970, but 1.24 and 1.11 on two
+// of the uniform ones, of 2200 0.995.  Ids 2 to 6, which are only forced, have
+// theirs alone.)
 constexpr TileCost kSimtTailNs[kSimtNumCfgs] = {
-    {1500.0f, 25.0f}, {2400.0f, 45.0f}, {2100.0f, 30.0f}, {2100.0f, 30.0f}, {2700.0f, 45.0f},
+    {1900.0f, 16.0f}, {2400.0f, 45.0f}, {2100.0f, 30.0f}, {2100.0f, 30.0f}, {2700.0f, 45.0f},
     {3400.0f, 70.0f}, {3400.0f, 70.0f}, {3664.0f, 120.0f}, {2400.0f, 22.5f}, {2100.0f, 20.5f}};
-// Id 0 has its 16 ns per k above kSimtShortK, or a few thin matrices of long K
-// take thin tiles, which end later than 16 x 16 ones (two of 8 x 512 x 4096: 93
-// us, 68 so; eight of 256 x 256 x 4096 147 and 157, 430 with the factors that
-// stood here first; 304 batches, those of long K among them, 0.985).
-template <int C>
-__host__ __device__ inline float simt_tail_ns(int K) {
-  constexpr TileCost t = kSimtTailNs[C];
-  constexpr TileCost beyond = {t.a_ns + (t.b_ns - 16.0f) * kSimtShortK, 16.0f};
-  return simt_tile_ns(K, C == 0 && K > kSimtShortK ? beyond : t);
-}
 // All tiles of a matrix.  A ragged edge's FMAs are skipped in steps of gm x gn
 // outputs, its copies are not.
 __host__ __device__ inline float simt_work_ns(int M, int N, int K, SimtCfg g, TileCost t) {
@@ -171,7 +157,7 @@ __host__ __device__ inline void simt_cand(int M, int N, int K, int force, SimtCa
   e->lat[C] = -1.0f;
   if ((force >= 0 ? C != force : !simt_auto_cfg(C, M, N)) || !simt_fits(M, N, g)) return;
   e->work[C] = simt_work_ns(M, N, K, g, t);
-  e->lat[C] = simt_tail_ns<C>(K);
+  e->lat[C] = simt_tile_ns(K, kSimtTailNs[C]);
 }
 template <int... C>
 __host__ __device__ inline void simt_cands_of(std::integer_sequence<int, C...>, int M, int N,
