@@ -82,10 +82,8 @@ constexpr int kPackK = 256;
 // thread issues all kPackK / 8 of its loads for a chunk before it stores, and
 // writes four consecutive k per store (rows are 16-byte aligned, so packed
 // writes are full vectors; the K tail and rows past M/N are masked).
-// At most 64 registers, so that four CTAs fit an SM (256 matrices of 16 to 256
-// in split TF32, whole call: 63.6 us where the compiler took 79, 61.1 so).
 template <int KIND, int SPLIT>
-__global__ void __launch_bounds__(256, 4) tc_pack_kernel(const TcPackParams p) {
+__global__ void __launch_bounds__(256) tc_pack_kernel(const TcPackParams p) {
   __shared__ __align__(16) float t[kPackK][33];
   pdl_trigger();
   pdl_wait();
@@ -201,12 +199,17 @@ __global__ void __launch_bounds__(256, 4) tc_pack_kernel(const TcPackParams p) {
       const int wk = (tid & 7) * 4;
       if (n >= rows) continue;
       const float* col = X + n * ldx;
+      // Always true here, but part of the loads' condition: without it the
+      // compiler takes 79 registers instead of 63 and a CTA less fits an SM (256
+      // matrices of 16 to 256 in split TF32, whole call: 63.6 us, 60.8 so; 61.1
+      // without it at 64 registers by launch bounds).
+      const bool vec = ((reinterpret_cast<uintptr_t>(col) & 15u) == 0);
       for (int k0 = 0; k0 < K; k0 += kPackK) {
         float x[kPackK / 32][4];
 #pragma unroll
         for (int h2 = 0; h2 < kPackK / 32; ++h2) {
           const int k = k0 + wk + 32 * h2;
-          if (k + 4 <= K) {
+          if (vec && k + 4 <= K) {
             const float4 f = *reinterpret_cast<const float4*>(col + k);
             x[h2][0] = f.x; x[h2][1] = f.y; x[h2][2] = f.z; x[h2][3] = f.w;
           } else {
