@@ -38,7 +38,9 @@
  * device pointers dA/dB/dC; the library owns its plans, their device
  * descriptors and workspace.  All device work is asynchronous on `stream`.
  * A plan may be executed on one stream at a time (its tile queue counter is
- * reset by the kernel itself at the end of each launch).
+ * reset by the kernel itself at the end of each launch), and its descriptors
+ * are uploaded on the stream it was created or updated on: order an execute on
+ * another stream behind that one, or it reads descriptors not yet there.
  */
 #ifndef BGEMM_GB300_H
 #define BGEMM_GB300_H
